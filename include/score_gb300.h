@@ -205,7 +205,10 @@ int  score_grain_counts(score_ctx* ctx, uint32_t* rxg_counts, uint32_t* defg_cou
  * from the start of the restart/reset to the end of the last score_run_until */
 /* Device phase times (total, grow, claim, commit, fill) and the algorithmic bytes are sums over
  * the TIMED steps: every timing_every-th step of a run (score_tune), timed_steps of them; the
- * steps in between run without phase events.  Host times and counts cover every step. */
+ * steps in between run without phase events.  Host times and counts cover every step.
+ * Steps of small fronts run inside one launch (k_steps_fused): their phases come from the device's
+ * clock, fill_ms with the infection attempts in it, grow_ms with the recycle list and the wins,
+ * commit_ms with the new cells; a batch's are those of its first running domain. */
 typedef struct score_timing {
     double total_ms;        /* device time of the step kernels */
     double grow_ms;         /* the fill update and the FullRX / recycle lists (k_grow_fill, k_grow_lists) */

@@ -33,6 +33,7 @@
 #include "../../include/score_gb300.h"
 #include "device_common.cuh"
 #include "growth_kernels.cuh"
+#include "fused_step.cuh"
 #include "host_model.h"
 #include "percolation.h"
 
@@ -430,7 +431,16 @@ struct score_ctx {
     HostBox* h_box = nullptr;          // pinned, device-mapped step mailbox
     HostBox* d_box = nullptr;          // its device address
     double* d_pforce = nullptr;
-    double* h_pforce = nullptr;            // pinned staging of the driving forces
+    double* h_pforce = nullptr;            // pinned staging of the driving forces: two buffers of ndefg, in turn
+    int pf_buf = 0;                        // the buffer with the newest
+    bool pf_pending = false;               // not on the device yet
+    // stepping inside one launch (k_steps_fused)
+    uint32_t fuse_seq = 1;                 // number of the next command
+    bool fuse_live = false;                // a launch steps this domain: driving forces go by its commands
+    bool pre_done = false;                 // pre_step ran for a step that no launch has taken yet
+    uint32_t pre_newnuc = 0;
+    uint32_t fuse_replay = 0;              // flags of a command that its launch left without seeing (kCmdReplay set)
+    FusePay fuse_sent{};                   // the payload the running launch has
     NucDue* h_due = nullptr;               // pinned staging of nuclei due during the run
     NucDue* d_due = nullptr;
     uint32_t* d_grid_init = nullptr;       // the loaded deformed grid (restart source)
@@ -489,7 +499,7 @@ struct score_ctx {
 
 void score_ctx::release_domain() {
     if (device >= 0) cudaSetDevice(device);
-    void* ptrs[] = {a.f[0].inc, a.f[1].inc, scratch.inc, a.f[0].mob, a.f[1].mob, scratch.mob, a.f[0].fill, a.f[0].comp, a.f[0].vel, a.f[0].defg, a.f[0].rxg, a.f[0].xyz, a.f[0].dir, a.f[0].full, a.f[0].recyc,
+    void* ptrs[] = {a.fuse, a.f[0].inc, a.f[1].inc, scratch.inc, a.f[0].mob, a.f[1].mob, scratch.mob, a.f[0].fill, a.f[0].comp, a.f[0].vel, a.f[0].defg, a.f[0].rxg, a.f[0].xyz, a.f[0].dir, a.f[0].full, a.f[0].recyc,
                     a.f[1].fill, a.f[1].comp, a.f[1].vel, a.f[1].defg, a.f[1].rxg, a.f[1].xyz, a.f[1].dir, a.f[1].full, a.f[1].recyc,
                     a.grid, a.claim, a.amask, a.ptab, a.defg_cnt, a.rxg_cnt, a.depleted, a.miss, a.tobm, a.ctcnt, a.fcell,
                     a.f[0].fmask, a.f[0].imask, a.f[0].tcnt, a.f[1].fmask, a.f[1].imask, a.f[1].tcnt,
@@ -575,6 +585,7 @@ public:
         cv_.notify_all();
         for (auto& t : th_) t.join();
     }
+    size_t size() const { return th_.size(); }
     // run f(0..n-1) on the workers and the calling thread; returns when all are done
     void run(int n, const std::function<void(int)>& f) {
         const uint64_t g = ++round_;
@@ -692,6 +703,12 @@ struct Engine {
         if (e == cudaSuccess) e = cudaMallocHost((void**)&h_args, (size_t)ndom * sizeof(DomainArgs));
         h_args_dev.assign((size_t)ndom, DomainArgs{});
         args_dirty = true;
+        int coop = 0;
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_steps_fused<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FuseShared));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_steps_fused<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FuseShared));
+        fuse = e == cudaSuccess && coop != 0;
+        fuse_sms = sms;
         return e == cudaSuccess ? SCORE_OK : SCORE_ERR_CUDA;
     }
     void drop_graph() {
@@ -720,12 +737,16 @@ struct Engine {
     void launch_sequence(int n);
     cudaError_t enqueue_step(int n, bool timed, int mode);
     int step(bool timed);
+    bool fused_ok() const;
+    int fused_session(double x_target, uint32_t max_steps, bool one, std::vector<uint32_t>& done);
     void balance_weights();
     int run_until(double x_target, uint32_t max_steps, uint32_t* steps_done);
     int autotune(double x_target, uint32_t max_steps, score_tune* out);
     void get_tune(score_tune* out) const;
     int set_tune(const score_tune* t);
     void mark_run_start() { cudaEventRecord(ev[5], stream); run_steps = 0; }
+    bool fuse = false;                 // cooperative launches of k_steps_fused are possible
+    int fuse_sms = 1;                  // blocks of one of them (batches share the SMs between their engines)
     bool sample_step() const { return cfg.timing_every > 0 && run_steps % (uint64_t)cfg.timing_every == 0; }
     int mark_run_end();
 };
@@ -763,6 +784,16 @@ namespace {
 template <class Body>
 void for_grains(score_ctx* c, Body body);
 
+// newest driving forces to the device, in stream order
+int flush_pforce(score_ctx* c) {
+    if (!c->pf_pending) return SCORE_OK;
+    const cudaError_t e = cudaMemcpyAsync(c->d_pforce, c->h_pforce + (size_t)c->pf_buf * c->ndefg, (size_t)c->ndefg * 8,
+                                          cudaMemcpyHostToDevice, c->stream);
+    if (e != cudaSuccess) return c->cuda_fail(e, "upload driving force");
+    c->pf_pending = false;
+    return SCORE_OK;
+}
+
 // Driving force per deformed grain, the grow step's p (SCORE_Kernel.cpp:4082), from `rho`
 // (whose version is `rho_ver`).  When it or the mobilities change, the front's velocity
 // factors are recomputed in the next grow.  The copy is stream-ordered after every launch
@@ -776,15 +807,16 @@ int upload_physics(score_ctx* c, const double* rho, uint64_t rho_ver) {
         return SCORE_OK;
     memcpy(c->pf_sig, sig, sizeof sig);
     c->pf_rho_version = rho_ver;
-    // new p per grain, straight into the pinned staging buffer (its last copy to the device
-    // finished before the step that just ended), noting whether any value changed
+    // new p per grain, straight into the pinned staging buffer that the device does not read (the last
+    // copy out of it finished before the step that just ended), noting whether any value changed
+    double* const h_new = c->h_pforce + (size_t)(c->pf_buf ^ 1) * c->ndefg;
     if (c->pforce_host.size() != c->ndefg) c->pforce_host.assign(c->ndefg, std::numeric_limits<double>::quiet_NaN());
     std::atomic<bool> pf_changed{false};
     for_grains(c, [&](size_t lo, size_t hi) {
         bool ch = false;
         for (size_t g = lo; g < hi; ++g) {
             const double v = c->ph.driving_force(rho[g]);
-            c->h_pforce[g] = v;
+            h_new[g] = v;
             if (v != c->pforce_host[g]) { c->pforce_host[g] = v; ch = true; }
         }
         if (ch) pf_changed.store(true);
@@ -793,9 +825,9 @@ int upload_physics(score_ctx* c, const double* rho, uint64_t rho_ver) {
     c->refresh = (c->refresh == 1 || !mob_same) ? 1 : 2;  // new mobilities need P again
     memcpy(c->mob_host, mob, sizeof mob);
     if (!pf_changed.load()) return SCORE_OK;
-    const cudaError_t e = cudaMemcpyAsync(c->d_pforce, c->h_pforce, (size_t)c->ndefg * 8, cudaMemcpyHostToDevice, c->stream);
-    if (e != cudaSuccess) return c->cuda_fail(e, "upload driving force");
-    return SCORE_OK;
+    c->pf_buf ^= 1;
+    c->pf_pending = true;
+    return c->fuse_live ? SCORE_OK : flush_pforce(c);
 }
 
 void set_step_args(score_ctx* c) {
@@ -1053,6 +1085,9 @@ int reset_state(score_ctx* c) {
     for (size_t k = 0; k < c->log_cells.size(); ++k) c->log_cells[k] = c->prm.logpoint_x[k] * (double)c->N;  // log_initialization, :60-62
     memset(&c->h_box->snap, 0, sizeof(DevState));
     c->running = false;
+    c->pre_done = false;
+    c->fuse_replay = 0;
+    c->pf_pending = false;
     c->trace.clear();
     c->rho = c->rho0;
     c->defg_cnt_host = c->defg_cnt_init_host;
@@ -1514,8 +1549,14 @@ int Engine::step(bool timed) {
     for (int i = 0; i < n; ++i) {
         score_ctx* c = dom[i];
         if (c->running) {
-            const int s = pre_step(c, &newnuc[i]);
+            const int s = c->pre_done ? SCORE_OK : pre_step(c, &c->pre_newnuc);
             if (s != SCORE_OK) return fail(s, c->err);
+            newnuc[i] = c->pre_newnuc;
+            c->pre_done = false;
+            if ((c->fuse_replay & kCmdForce) &&  // the forces of a command that no launch took
+                cudaMemcpyAsync(c->d_pforce, c->h_box->fuse.pay.pf_src, (size_t)c->ndefg * 8, cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
+                return fail(SCORE_ERR_CUDA, "upload driving force");
+            c->fuse_replay = 0;
             ++nrun;
         } else {
             c->a.active = 0;
@@ -1551,7 +1592,7 @@ int Engine::step(bool timed) {
             score_ctx* c = dom[i];
             if (!c->running) return;
             cudaSetDevice(device);  // the calling thread may be a worker
-            status[i] = physics_ahead(c);
+            status[i] = c->ahead ? flush_pforce(c) : physics_ahead(c);
         };
         if (n >= 4) {
             workers(15);
@@ -1626,23 +1667,345 @@ int Engine::mark_run_end() {
     return SCORE_OK;
 }
 
+// ------------------------------------------------------------------ many steps in one launch
+namespace {
+
+// Slots of a domain's front up to which its steps run inside one launch.  A fused step saves the separate
+// kernels' fixed cost (about 50 us) but streams a large front at half their occupancy.  Measured per run,
+// limits of 0 / 1 / 2 / 4 / 8 M slots: FP64 384^3 rolled sheet 68.2 / 68.5 / 68.2 / 69.2 / 83.5 ms, FP64 512^3
+// 116.9 / 115.8 / 114.5 / 114.8 / 115.3, FP32 384^3 with recovery 210.6 / 180.1 / 172.5 / 151.4 / 149.6, batch of
+// 12 FP64 84.5 / 71.0 / 64.0 / 64.9 / 64.5.
+constexpr uint64_t kFuseSlots = (uint64_t)kFuseMaxTiles * kFuseTile / 2;
+
+uint32_t fuse_tiles(const score_ctx* c) {
+    return (c->next_never[0] + kFuseTile - 1) / kFuseTile + (c->next_never[1] + kFuseTile - 1) / kFuseTile;
+}
+
+FusePay fuse_pay(const score_ctx* c) {
+    FusePay p{};
+    const DomainArgs& a = c->a;
+    p.mLAGB = a.mLAGB; p.mHAGB = a.mHAGB; p.mGS = a.mGS; p.mRH = a.mRH;
+    p.dt = a.dt; p.cinv = a.cinv; p.dtc32 = a.dtc32;
+    p.ans_idx = a.ans_idx; p.ans_val = a.ans_val;
+    p.pf_src = c->h_pforce + (size_t)c->pf_buf * c->ndefg;
+    return p;
+}
+
+uint32_t fuse_flags(const score_ctx* c) {
+    const DomainArgs& a = c->a;
+    return (a.dt_changed ? kCmdDtChanged : 0u) | (a.spec ? kCmdSpec : 0u) |
+           (a.refresh == 1 ? kCmdRefresh1 : a.refresh == 2 ? kCmdRefresh2 : 0u);
+}
+
+inline void fuse_store(uint32_t* p, uint32_t v) { __atomic_store_n(p, v, __ATOMIC_RELEASE); }
+inline uint32_t fuse_load(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_ACQUIRE); }
+
+// whether the next step needs the stream before it starts: nuclei due, a defragmentation
+bool fuse_needs_stream(const score_ctx* c) {
+    if (c->nuc_pos < c->nuc_order.size() && c->tincub[c->nuc_order[c->nuc_pos]] <= c->ph.t) return true;
+    return c->prm.defragmentation && c->defrag_cnt < c->prm.n_defrag && c->Xcells >= c->prm.defrag_x[c->defrag_cnt] * (double)c->N;
+}
+
+// one domain of a session, as its host thread sees it
+struct FuseServe {
+    score_ctx* c = nullptr;
+    size_t i = 0;
+    uint32_t blocks = 0;
+    bool open = false;      // its group steps, or was told to
+    bool deferred = false;  // posted, but its post step needs the stream: after the launch
+    int status = SCORE_OK;
+    uint32_t steps = 0, timed = 0;
+    uint32_t word = 0;      // its last command
+    double bytes = 0.0, sbytes = 0.0, fill = 0.0, res = 0.0, com = 0.0, post = 0.0;
+};
+
+}  // namespace
+
+// Steps run inside one launch while every running domain's front is small; the launch configuration's
+// direct launches (use_graph 0, the autotuner) keep the separate kernels.
+bool Engine::fused_ok() const {
+    if (!fuse || !use_graph) return false;
+    uint64_t nrun = 0, tiles = 0;
+    for (const score_ctx* c : dom) {
+        if (!c->running) continue;
+        ++nrun;
+        tiles += fuse_tiles(c);
+        if ((uint64_t)c->next_never[0] + c->next_never[1] > kFuseSlots) return false;
+    }
+    // a domain's blocks follow its share of the tiles: kFuseMaxLocal tiles a block with room to grow
+    return nrun > 0 && nrun < (uint64_t)fuse_sms && tiles + 4 * nrun <= (kFuseMaxLocal / 2) * ((uint64_t)fuse_sms - nrun);
+}
+
+// One launch that steps every running domain until it meets its stop rule, needs the stream (nuclei due, a
+// logged step, a defragmentation, requests beyond the mailbox) or the launch has run for a while: other
+// work of the device gets its turn then.  `one`: a single step.  done[i]: steps of domain i in this run.
+int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::vector<uint32_t>& done) {
+    cudaSetDevice(device);
+    const auto t0 = std::chrono::steady_clock::now();
+    const int n = (int)dom.size();
+    std::vector<FuseServe> sv;
+    FuseMap map{};
+    uint64_t work = 0;
+    for (int i = 0; i < n; ++i) {
+        score_ctx* c = dom[i];
+        if (!c->running) { c->a.active = 0; h_args[i] = c->a; continue; }
+        const int s = c->pre_done ? SCORE_OK : pre_step(c, &c->pre_newnuc);
+        if (s != SCORE_OK) return fail(s, c->err);
+        c->pre_done = true;
+        h_args[i] = c->a;
+        FuseServe f;
+        f.c = c; f.i = (size_t)i;
+        sv.push_back(f);
+        work += 2ull * fuse_tiles(c) + 8;
+    }
+    const auto t_pre = std::chrono::steady_clock::now();
+    tm.pre_ms += std::chrono::duration<double, std::milli>(t_pre - t0).count();
+    // blocks in proportion to the fronts, at least one a domain, no more than tiles a front may have soon
+    uint32_t total = 0;
+    {
+        const uint32_t spare = (uint32_t)fuse_sms - (uint32_t)sv.size();
+        size_t k = 0;
+        for (int i = 0; i < n; ++i) {
+            map.first[i] = (uint16_t)total;
+            if (k < sv.size() && sv[k].i == (size_t)i) {
+                const uint32_t want = 2 * fuse_tiles(sv[k].c) + 8;
+                sv[k].blocks = std::min(want, 1u + (uint32_t)((uint64_t)spare * want / work));
+                total += sv[k].blocks;
+                map.seq[i] = sv[k].c->fuse_seq;
+                ++k;
+            }
+        }
+        map.first[n] = (uint16_t)total;
+        map.ndom = (uint32_t)n;
+    }
+    cudaError_t e = cudaSuccess;
+    if (args_dirty || memcmp(h_args, h_args_dev.data(), (size_t)n * sizeof(DomainArgs)) != 0) {
+        e = cudaMemcpyAsync(d_args, h_args, (size_t)n * sizeof(DomainArgs), cudaMemcpyHostToDevice, stream);
+        memcpy(h_args_dev.data(), h_args, (size_t)n * sizeof(DomainArgs));
+        args_dirty = false;
+    }
+    for (FuseServe& f : sv) {
+        score_ctx* c = f.c;
+        if (c->fuse_replay) {
+            f.word = c->fuse_replay & ((1u << kCmdShift) - 1u);
+            c->fuse_sent = c->h_box->fuse.pay;
+        } else {
+            f.word = fuse_flags(c);
+            c->fuse_sent = fuse_pay(c);
+        }
+        c->fuse_replay = 0;
+        f.word |= (c->fuse_seq << kCmdShift) | (one ? kCmdLast : 0u);
+        fuse_store(&c->h_box->fuse.cmd, f.word);
+        c->fuse_live = true;
+        f.open = true;
+    }
+    if (e == cudaSuccess) {
+        void* args[] = {(void*)&map, (void*)&base};
+        const void* k = fp32 ? (const void*)k_steps_fused<true> : (const void*)k_steps_fused<false>;
+        e = cudaLaunchCooperativeKernel(k, dim3(total), dim3(kFuse), args, sizeof(FuseShared), stream);
+    }
+    if (e != cudaSuccess) {
+        for (FuseServe& f : sv) f.c->fuse_live = false;
+        if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources) {
+            cudaGetLastError();
+            fuse = false;  // the separate kernels from now on
+            return SCORE_OK;
+        }
+        for (score_ctx* c : dom) c->failed = true;
+        return fail(SCORE_ERR_CUDA, std::string("growth steps: ") + cudaGetErrorString(e));
+    }
+    launches += 1;
+    std::atomic<bool> stop{false};
+    const double bpu = fp32 ? 21.0 : 25.0;
+    const uint64_t sample0 = run_steps;
+    auto timed_step = [&](const FuseServe& f) {
+        return cfg.timing_every > 0 && (sample0 + f.steps) % (uint64_t)cfg.timing_every == 0;
+    };
+    auto leave = [&](FuseServe& f) {  // the posted step's group leaves the launch
+        score_ctx* c = f.c;
+        f.open = false;
+        if (one) return;  // it has left
+        fuse_store(&c->h_box->fuse.cmd, (c->fuse_seq << kCmdShift) | kCmdLeave);
+        c->fuse_seq = (c->fuse_seq + 1) & kCmdSeqMask;
+    };
+    // after the post of a step: the host's part of it, and the next command
+    auto finish_step = [&](FuseServe& f) -> int {
+        score_ctx* c = f.c;
+        const FuseHost& h = c->h_box->fuse;
+        const auto p0 = std::chrono::steady_clock::now();
+        const bool is_timed = timed_step(f);
+        if (is_timed) {
+            f.timed++;
+            f.fill += 1e-6 * h.phase_ns[0]; f.res += 1e-6 * h.phase_ns[1]; f.com += 1e-6 * h.phase_ns[2];
+        }
+        c->pre_done = false;
+        const int s = post_step(c, c->pre_newnuc, nullptr);
+        if (s != SCORE_OK) return s;
+        if (is_timed || sv.size() > 1) {
+            f.bytes += bpu * (double)c->last.Sv;
+            f.sbytes += 120.0 * (double)c->last.n_full + 37.0 * (double)c->last.n_new;
+        }
+        if (!c->ans_idx.empty() && c->ans_idx.size() <= kBoxMiss) {
+            memcpy(c->h_box->ans_idx, c->ans_idx.data(), c->ans_idx.size() * 8);
+            memcpy(c->h_box->ans_val, c->ans_val.data(), c->ans_val.size() * 8);
+            c->a.ans_idx = c->d_box->ans_idx;
+            c->a.ans_val = c->d_box->ans_val;
+        }
+        f.steps++;
+        done[f.i]++;
+        if (!one) c->trace.push_back(c->last);
+        f.post += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - p0).count();
+        return SCORE_OK;
+    };
+    // one look at a domain's mailbox; false when there was nothing new
+    auto poll = [&](FuseServe& f) -> bool {
+        score_ctx* c = f.c;
+        FuseHost& h = c->h_box->fuse;
+        const uint32_t seq = c->fuse_seq;
+        if (fuse_load(&h.post) != seq) {
+            if (fuse_load(&h.left) != seq) return false;
+            f.open = false;  // the group left before it saw the command: the next launch takes the step
+            c->fuse_seq = (seq + 1) & kCmdSeqMask;
+            c->fuse_replay = (f.word & ((1u << kCmdShift) - 1u) & ~kCmdLast) | kCmdReplay;
+            return true;
+        }
+        c->fuse_seq = (seq + 1) & kCmdSeqMask;
+        const DevState& hs = c->h_box->snap;
+        if (hs.err || hs.nmiss > kBoxMiss || hs.ndepleted > kBoxDep) {
+            f.deferred = true;
+            stop.store(true, std::memory_order_relaxed);
+            leave(f);
+            return true;
+        }
+        const size_t logged = c->log_info.size();
+        f.status = finish_step(f);
+        const double xt = x_target < 0 ? c->prm.xmax : x_target;
+        const bool needs = f.status == SCORE_OK && (c->log_info.size() != logged || fuse_needs_stream(c) ||
+                           (uint64_t)c->next_never[0] + c->next_never[1] > kFuseSlots || fuse_tiles(c) > kFuseMaxLocal * f.blocks);
+        if (f.status != SCORE_OK || needs) stop.store(true, std::memory_order_relaxed);
+        if (f.status != SCORE_OK || needs || one || domain_done(c, xt) || (max_steps && done[f.i] >= max_steps) ||
+            stop.load(std::memory_order_relaxed)) {
+            leave(f);
+            return true;
+        }
+        f.status = pre_step(c, &c->pre_newnuc);  // no nuclei, no defragmentation: arguments only
+        if (f.status != SCORE_OK) { stop.store(true, std::memory_order_relaxed); leave(f); return true; }
+        c->pre_done = true;
+        uint32_t w = (c->fuse_seq << kCmdShift) | fuse_flags(c);
+        const FusePay pay = fuse_pay(c);
+        if (c->pf_pending) { w |= kCmdForce | kCmdPayload; c->pf_pending = false; }
+        if (memcmp(&pay, &c->fuse_sent, sizeof pay) != 0) w |= kCmdPayload;
+        if (w & kCmdPayload) { h.pay = pay; c->fuse_sent = pay; }
+        f.word = w;
+        fuse_store(&h.cmd, w);
+        f.status = physics_ahead(c);  // while the group steps
+        if (f.status != SCORE_OK) stop.store(true, std::memory_order_relaxed);
+        return true;
+    };
+    // serve domains first, first + every, ... until all their groups have left
+    auto serve = [&](size_t first, size_t every) {
+        cudaSetDevice(device);  // the calling thread may be a worker
+        for (size_t k = first; k < sv.size(); k += every) {
+            if (!sv[k].c->ahead) sv[k].status = physics_ahead(sv[k].c);
+            if (sv[k].status != SCORE_OK) stop.store(true, std::memory_order_relaxed);
+        }
+        uint32_t idle = 0;
+        for (;;) {
+            bool open = false, any = false;
+            for (size_t k = first; k < sv.size(); k += every) {
+                if (!sv[k].open) continue;
+                any |= poll(sv[k]);
+                open |= sv[k].open;
+            }
+            if (!open) return;
+            if (any) idle = 0;
+            if ((any || (++idle & 0xFFFu) == 0) && std::chrono::steady_clock::now() - t_pre > std::chrono::milliseconds(2))
+                stop.store(true, std::memory_order_relaxed);
+            if (any || (idle & 0xFFFFu) != 0) continue;
+            // long silence: has the launch ended (an error, or a wait on the device that gave up)?
+            const cudaError_t q = cudaStreamQuery(stream);
+            if (q == cudaErrorNotReady) continue;
+            for (size_t k = first; k < sv.size(); k += every) {
+                if (!sv[k].open || poll(sv[k])) continue;  // its posts came before its end
+                sv[k].open = false;
+                sv[k].c->failed = true;
+                sv[k].status = q != cudaSuccess ? sv[k].c->cuda_fail(q, "growth steps")
+                                                : sv[k].c->fail(SCORE_ERR_TIMEOUT, "a bounded device wait gave up");
+            }
+        }
+    };
+    const size_t threads = std::min<size_t>(sv.size(), sv.size() > 1 ? 16 : 1);
+    if (threads > 1) {
+        WorkerPool& p = workers(15);
+        const size_t every = std::min<size_t>(threads, p.size() + 1);
+        p.run((int)every, [&](int w) { serve((size_t)w, every); });
+    } else {
+        serve(0, 1);
+    }
+    if (!one) {
+        e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) {
+            for (score_ctx* c : dom) c->failed = true;
+            return fail(SCORE_ERR_CUDA, std::string("growth steps: ") + cudaGetErrorString(e));
+        }
+    }
+    bool staged = false;
+    int status = SCORE_OK;
+    for (FuseServe& f : sv) {
+        score_ctx* c = f.c;
+        c->fuse_live = false;
+        if (f.deferred && f.status == SCORE_OK) {
+            f.status = finish_step(f);
+            staged |= c->ans_idx.size() > kBoxMiss;
+        }
+        if (f.status == SCORE_OK && !c->fuse_replay) f.status = flush_pforce(c);
+        if (f.status != SCORE_OK && status == SCORE_OK) { status = f.status; fail(status, c->err); }
+        tm.weights_ms += c->weights_ms;
+        c->weights_ms = 0.0;
+    }
+    if (status == SCORE_OK && staged) status = stage_answers();
+    // the first domain's steps and phases stand for the launch's; bytes are every domain's in the timed share
+    const FuseServe& f0 = sv[0];
+    double bytes = 0.0, sbytes = 0.0;
+    for (const FuseServe& f : sv) { bytes += f.bytes; sbytes += f.sbytes; }
+    const double share = sv.size() == 1 ? 1.0 : f0.steps ? (double)f0.timed / f0.steps : 0.0;
+    tm.fill_ms += f0.fill; tm.grow_ms += f0.fill + f0.res; tm.commit_ms += f0.com; tm.total_ms += f0.fill + f0.res + f0.com;
+    tm.timed_steps += f0.timed;
+    tm.grow_launches += f0.steps;
+    tm.grow_bytes += bytes * share;
+    tm.step_bytes += (bytes + sbytes) * share;
+    run_steps += f0.steps;
+    const double wall = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    double post = 0.0;
+    for (const FuseServe& f : sv) post = std::max(post, f.post);
+    tm.host_ms += wall;
+    tm.post_ms += post;
+    tm.wait_ms += std::max(0.0, wall - post - std::chrono::duration<double, std::milli>(t_pre - t0).count());
+    return status;
+}
+
 // Step every domain until each meets its stop rule (X > x_target, time or step limits);
 // a domain that stops leaves the launches, the others go on.  Each domain's per-step
 // stats are kept in its trace.
 int Engine::run_until(double x_target, uint32_t max_steps, uint32_t* steps_done) {
     uint32_t k = 0;
+    std::vector<uint32_t> done(dom.size(), 0);  // steps of each domain
     for (;;) {
         int nrun = 0;
-        for (score_ctx* c : dom) {
+        for (size_t i = 0; i < dom.size(); ++i) {
+            score_ctx* c = dom[i];
             const double xt = x_target < 0 ? c->prm.xmax : x_target;
-            c->running = c->loaded && !c->failed && !domain_done(c, xt);
+            c->running = c->loaded && !c->failed && !domain_done(c, xt) && !(max_steps && done[i] >= max_steps);
             nrun += c->running;
         }
-        if (nrun == 0 || (max_steps && k >= max_steps)) break;
-        const int s = step(sample_step());
+        if (nrun == 0) break;
+        const bool fused = fused_ok();
+        const int s = fused ? fused_session(x_target, max_steps, false, done) : step(sample_step());
+        if (!fused && s == SCORE_OK)
+            for (size_t i = 0; i < dom.size(); ++i)
+                if (dom[i]->running) { dom[i]->trace.push_back(dom[i]->last); ++done[i]; }
+        k = done.empty() ? 0 : *std::max_element(done.begin(), done.end());
         if (s != SCORE_OK) { if (steps_done) *steps_done = k; return s; }
-        for (score_ctx* c : dom) if (c->running) c->trace.push_back(c->last);
-        ++k;
     }
     for (score_ctx* c : dom) c->running = false;
     if (steps_done) *steps_done = k;
@@ -2024,8 +2387,10 @@ int score_load_domain(score_ctx* c, const uint32_t* grid, const double* defg_qua
         if (e == cudaSuccess) e = dalloc(&a.depleted, ndefg);
         if (e == cudaSuccess) e = dalloc(&a.miss, a.misscap);
         if (e == cudaSuccess) e = dalloc(&c->d_state, 1);
+        if (e == cudaSuccess) e = dalloc(&a.fuse, 1);
+        if (e == cudaSuccess) e = cudaMemsetAsync(a.fuse, 0, sizeof(FuseDom), c->stream);
         if (e == cudaSuccess) e = dalloc(&c->d_pforce, ndefg);
-        if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_pforce, std::max<size_t>(ndefg, 1) * 8);
+        if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_pforce, std::max<size_t>(ndefg, 1) * 16);
         if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_due, kDueMax * sizeof(NucDue));
         if (e == cudaSuccess) e = dalloc(&c->d_due, kDueMax);
         if (e == cudaSuccess) e = dalloc(&c->d_u32tmp, 64);
@@ -2084,7 +2449,8 @@ int score_step(score_ctx* c, score_step_stats* out) {
     if (!c->loaded) return c->fail(SCORE_ERR_STATE, "no domain loaded");
     if (c->failed) return SCORE_ERR_STATE;  // a device error left the front lists undefined
     c->running = true;
-    const int s = c->eng->step(c->eng->sample_step());
+    std::vector<uint32_t> done(1, 0);
+    const int s = c->eng->fused_ok() ? c->eng->fused_session(2.0, 1, true, done) : c->eng->step(c->eng->sample_step());
     c->running = false;
     if (s != SCORE_OK) { if (c->err.empty()) c->err = c->eng->err; return s; }
     if (out) *out = c->last;
@@ -2270,6 +2636,7 @@ int score_batch_create(score_batch** out, const score_params* params, uint32_t n
         const int si = E.init(device, (int)count[g]);
         if (si != SCORE_OK) { delete b; return si; }
         E.fp32 = params[0].precision == SCORE_PRECISION_FP32_KAHAN;
+        E.fuse_sms = std::max(1, E.sms / (int)G);  // the groups' launches run side by side
         E.pool_threads = std::max(1u, (hw - 1) / G);
     }
     for (uint32_t i = 0; i < n; ++i) {

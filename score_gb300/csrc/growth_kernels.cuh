@@ -81,6 +81,7 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t n, const FastDiv& f) {
 }
 
 struct HostBox;
+struct FuseDom;
 
 struct DomainArgs {
     DFront f[2];
@@ -114,6 +115,7 @@ struct DomainArgs {
                                         // order: table indices (kMissVoid = none), device view of pinned memory
     const double* ans_val;
     HostBox* box;               // device view of the domain's mailbox
+    FuseDom* fuse;              // barrier and word of the group that steps the domain inside one launch
     double mLAGB, mHAGB, mGS, mRH, dt, cinv;
     float dtc32;
     int32_t spec;               // few INACTIVE slots last step: k_grow_fill loads every slot's data with its
@@ -370,15 +372,14 @@ __device__ __forceinline__ void tile_masks(const DFront& fr, uint32_t tile, uint
     }
 }
 
-// returns the thread's ACTIVE slots (the Sv share)
+// The fill update of a thread's ITEMS slots base + 32 k of a list of n slots (a warp owns 32 ITEMS
+// consecutive slots): act bit k is set where item k's slot is ACTIVE, fullbits bit k where its cell is
+// full.  Returns the thread's ACTIVE slots (the Sv share).
 template <bool FP32, int REFRESH, int ITEMS>
-__device__ __forceinline__ uint32_t grow_tile(const DomainArgs& a, int L, uint32_t tile, uint32_t n) {
-    using S = GrowShape<ITEMS>;
-    const DFront& fr = a.f[L];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // each warp owns 32 * ITEMS consecutive slots of the tile: no block barrier, warps run apart
-    const uint32_t base = tile * S::kTile + (uint32_t)warp * 32u * ITEMS + (uint32_t)lane;
-    uint32_t sv = 0, act = 0;  // act bit k: item k's slot is ACTIVE
+__device__ __forceinline__ uint32_t grow_items(const DomainArgs& a, const DFront& fr, uint32_t base, uint32_t n, uint32_t& act,
+                                               uint32_t& fullbits) {
+    uint32_t sv = 0;
+    act = 0;
     uint8_t d[ITEMS];
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
@@ -386,7 +387,7 @@ __device__ __forceinline__ uint32_t grow_tile(const DomainArgs& a, int L, uint32
         d[k] = slot < n ? fr.dir[slot] : kInactive;
         if (d[k] != kInactive) act |= 1u << k;
     }
-    uint32_t fullbits = 0;  // bit k: item k's cell is full
+    fullbits = 0;
     if (!FP32 && REFRESH == 3) {
         double w[ITEMS], fill[ITEMS];
 #pragma unroll
@@ -615,7 +616,18 @@ __device__ __forceinline__ uint32_t grow_tile(const DomainArgs& a, int L, uint32
             }
         }
     }
-    tile_masks<ITEMS>(fr, tile, base, n, act, fullbits);
+    return sv;
+}
+
+// one grow tile of list L by the whole block; returns the thread's ACTIVE slots
+template <bool FP32, int REFRESH, int ITEMS>
+__device__ __forceinline__ uint32_t grow_tile(const DomainArgs& a, int L, uint32_t tile, uint32_t n) {
+    using S = GrowShape<ITEMS>;
+    // each warp owns 32 * ITEMS consecutive slots of the tile: no block barrier, warps run apart
+    const uint32_t base = tile * S::kTile + (threadIdx.x >> 5) * 32u * ITEMS + (threadIdx.x & 31u);
+    uint32_t act, fullbits;
+    const uint32_t sv = grow_items<FP32, REFRESH, ITEMS>(a, a.f[L], base, n, act, fullbits);
+    tile_masks<ITEMS>(a.f[L], tile, base, n, act, fullbits);
     return sv;
 }
 
@@ -1427,10 +1439,35 @@ __device__ __forceinline__ bool lookup_p(const DomainArgs& a, uint32_t rxg, uint
 // the host needs one stream synchronization per step and no copies.
 constexpr uint32_t kBoxMiss = 16384;
 constexpr uint32_t kBoxDep = 16384;
+// The host's word and answers to a group of blocks that steps a domain inside one launch
+// (k_steps_fused): what changes between steps, and the group's posts.
+struct FusePay {
+    double mLAGB, mHAGB, mGS, mRH, dt, cinv;
+    const unsigned long long* ans_idx;
+    const double* ans_val;
+    const double* pf_src;      // device view of the pinned driving forces
+    float dtc32;
+    uint32_t pad[5];
+};
+static_assert(sizeof(FusePay) % 4 == 0, "copied as words");
+
+struct FuseHost {
+    uint32_t cmd;              // host -> device
+    uint32_t pad0[31];
+    FusePay pay;               // host -> device, before cmd
+    uint32_t pad2[8];
+    uint32_t post;             // device -> host: step number whose record is in the mailbox
+    uint32_t left;             // device -> host: step number after which the group left on its own
+    uint32_t phase_ns[4];      // of the posted step: A, B, C, all
+    uint32_t pad1[26];
+};
 struct HostBox {
+    FuseHost fuse;
     DevState snap;
     unsigned long long miss[kBoxMiss];
     uint32_t depleted[kBoxDep];
+    unsigned long long ans_idx[kBoxMiss];   // weights the host computed for the last step's requests
+    double ans_val[kBoxMiss];
 };
 
 // The end of a domain's step, by one block: advances the high-water marks, posts the step to the
@@ -1565,6 +1602,71 @@ __device__ __forceinline__ void flush_new(const DomainArgs& a, double pmax, uint
     }
 }
 
+// per-grain cell counts of a warp's recrystallized cells (rx grain rs, deformed grain gs): one atomic per
+// grain and warp (full cells of one grain tend to finish together); every lane takes part
+__device__ __forceinline__ void count_full(const DomainArgs& a, bool has, uint32_t rs, uint32_t gs) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t act = __ballot_sync(0xFFFFFFFFu, has);
+    const uint32_t mr = __match_any_sync(0xFFFFFFFFu, has ? rs : 0xFFFFFFFFu) & act;
+    const uint32_t mg = __match_any_sync(0xFFFFFFFFu, has ? gs : 0xFFFFFFFFu) & act;
+    if (has && (__ffs(mr) - 1) == lane) atomicAdd(&a.rxg_cnt[rs], (uint32_t)__popc(mr));
+    if (has && (__ffs(mg) - 1) == lane) {
+        const uint32_t k = (uint32_t)__popc(mg);
+        const uint32_t old = atomicSub(&a.defg_cnt[gs], k);
+        if (old == k) {
+            const uint32_t q = atomicAdd(&a.st->ndepleted, 1u);
+            if (q < a.ndefg) a.depleted[q] = gs;
+        }
+    }
+}
+
+// A newly infected cell tgt (deformed grain gt until now) takes slot ns of list `dst`: overshoot `over` of the
+// full cell scaled by the direction's class, infector code of direction d, rx grain rs, and its mobility
+// weight and cached velocity factor (or a tag for the host's answer).
+template <bool FP32>
+__device__ __forceinline__ void new_cell(const DomainArgs& a, const DFront& dst, uint32_t ns, uint32_t tgt, uint32_t gt, uint32_t rs,
+                                         double over, int d, double& pmax, uint32_t& ntag) {
+    const double pf = a.pforce[gt];  // in flight together with the weight's load
+    const int cls = c_cls[d];
+    if (!FP32) {
+        const double fac = cls == 1 ? 0.0682 : (cls == 2 ? 0.0542 : 0.0484);
+        ((double*)dst.fill)[ns] = __dmul_rn(over, fac);
+    } else {
+        const float fac = cls == 1 ? 0.0682f : (cls == 2 ? 0.0542f : 0.0484f);
+        ((float*)dst.fill)[ns] = (float)over * fac;
+        dst.comp[ns] = 0.0f;
+    }
+    dst.defg[ns] = gt;
+    dst.rxg[ns] = rs;
+    dst.xyz[ns] = tgt;
+    a.grid[tgt] = 4096002000u;  // CURRENTLY_INFECTED
+    a.claim[tgt] = kClaimFree;
+    // mobility weight and cached velocity factor of the new cell
+    double P = 0.0;
+    uint32_t tag = 0;
+    if (lookup_p(a, rs, gt, P, tag)) {
+        const double mo = mobility(a, P);
+        dst.mob[ns] = mo;
+        const double v = velocity_from_force(mo, pf, c_code[d]);
+        if (!FP32) {
+            // the increment with this step's dt: valid next step unless dt changes, when
+            // k_grow_fill recomputes every increment from vel anyway
+            ((double*)dst.vel)[ns] = v;
+            dst.inc[ns] = __double_as_longlong(v) >= 0 ? __dmul_rn(__dmul_rn(v, a.dt), a.cinv) : v;
+        } else {
+            ((float*)dst.vel)[ns] = (float)v;
+        }
+        dst.dir[ns] = c_code[d];
+        if (P > pmax) pmax = P;
+    } else {
+        // vel holds the answer tag until the next k_grow_fill
+        if (!FP32) ((unsigned long long*)dst.vel)[ns] = tag;
+        else ((uint32_t*)dst.vel)[ns] = tag;
+        dst.dir[ns] = c_code[d] | kStale | kPend;
+        ++ntag;
+    }
+}
+
 template <bool FP32, bool ONE>
 __global__ void __launch_bounds__(kBlock, ONE ? 4 : 3) k_commit(int base, int ndom, uint32_t grow_tile) {
     __shared__ uint32_t s_pre[kMaxSegs + 1];
@@ -1669,46 +1771,7 @@ __global__ void __launch_bounds__(kBlock, ONE ? 4 : 3) k_commit(int base, int nd
             const uint32_t ns = r < nrec ? dst.recyc[r] : a.st->next_never[D] + (r - nrec);
             if (ns >= dst.cap) { atomicOr(&a.st->err, kErrCapacity); continue; }
             if (D == 1 && a.border_policy == 0 && r >= nrec && ns >= a.border_ref_cap) atomicOr(&a.st->err, kErrBorderRef);
-            const double pf = a.pforce[gt];  // in flight together with the weight's load
-            const int cls = c_cls[d];
-            if (!FP32) {
-                const double fac = cls == 1 ? 0.0682 : (cls == 2 ? 0.0542 : 0.0484);
-                ((double*)dst.fill)[ns] = __dmul_rn(s_over[t], fac);
-            } else {
-                const float fac = cls == 1 ? 0.0682f : (cls == 2 ? 0.0542f : 0.0484f);
-                ((float*)dst.fill)[ns] = (float)s_over[t] * fac;
-                dst.comp[ns] = 0.0f;
-            }
-            const uint32_t rs = s_rsrc[t];
-            dst.defg[ns] = gt;
-            dst.rxg[ns] = rs;
-            dst.xyz[ns] = tgt;
-            a.grid[tgt] = 4096002000u;  // CURRENTLY_INFECTED
-            a.claim[tgt] = kClaimFree;
-            // mobility weight and cached velocity factor of the new cell
-            double P = 0.0;
-            uint32_t tag = 0;
-            if (lookup_p(a, rs, gt, P, tag)) {
-                const double mo = mobility(a, P);
-                dst.mob[ns] = mo;
-                const double v = velocity_from_force(mo, pf, c_code[d]);
-                if (!FP32) {
-                    // the increment with this step's dt: valid next step unless dt changes, when
-                    // k_grow_fill recomputes every increment from vel anyway
-                    ((double*)dst.vel)[ns] = v;
-                    dst.inc[ns] = __double_as_longlong(v) >= 0 ? __dmul_rn(__dmul_rn(v, a.dt), a.cinv) : v;
-                } else {
-                    ((float*)dst.vel)[ns] = (float)v;
-                }
-                dst.dir[ns] = c_code[d];
-                if (P > pmax) pmax = P;
-            } else {
-                // vel holds the answer tag until the next k_grow_fill
-                if (!FP32) ((unsigned long long*)dst.vel)[ns] = tag;
-                else ((uint32_t*)dst.vel)[ns] = tag;
-                dst.dir[ns] = c_code[d] | kStale | kPend;
-                ++ntag;
-            }
+            new_cell<FP32>(a, dst, ns, tgt, gt, s_rsrc[t], s_over[t], d, pmax, ntag);
         }
         if (f < F) {
             // the full cell is now recrystallized
@@ -1718,23 +1781,7 @@ __global__ void __launch_bounds__(kBlock, ONE ? 4 : 3) k_commit(int base, int nd
             if (!FP32) ((double*)src.fill)[slot] = 0.0;
             else { ((float*)src.fill)[slot] = 0.0f; src.comp[slot] = 0.0f; }
         }
-        // per-grain cell counts: one atomic per grain and warp (full cells of one grain
-        // tend to finish together)
-        {
-            const bool has = f < F;
-            const uint32_t act = __ballot_sync(0xFFFFFFFFu, has);
-            const uint32_t mr = __match_any_sync(0xFFFFFFFFu, has ? rsrc : 0xFFFFFFFFu) & act;
-            const uint32_t mg = __match_any_sync(0xFFFFFFFFu, has ? gsrc : 0xFFFFFFFFu) & act;
-            if (has && (__ffs(mr) - 1) == lane) atomicAdd(&a.rxg_cnt[rsrc], (uint32_t)__popc(mr));
-            if (has && (__ffs(mg) - 1) == lane) {
-                const uint32_t k = (uint32_t)__popc(mg);
-                const uint32_t old = atomicSub(&a.defg_cnt[gsrc], k);
-                if (old == k) {
-                    const uint32_t q = atomicAdd(&a.st->ndepleted, 1u);
-                    if (q < a.ndefg) a.depleted[q] = gsrc;
-                }
-            }
-        }
+        count_full(a, f < F, rsrc, gsrc);
         __syncthreads();
     }
     if (cur >= 0) flush_new(c_args[base + cur], pmax, ntag);
