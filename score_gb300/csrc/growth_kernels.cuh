@@ -83,6 +83,15 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t n, const FastDiv& f) {
 struct HostBox;
 struct FuseDom;
 
+struct WeightClass {            // what the classification needs of the parameters
+    int32_t model;              // SCORE_MOBILITY_*; 0: no classification
+    float cos_lagb;             // cos(7.5 deg)
+    float cos_lo, cos_hi;       // cos of half of 30 and 50 deg: |angle - 40 deg| beyond 10 deg needs no axis
+    float cos_dev;              // cos(5 deg)
+    float cos_sat;              // cos of half the angle from which the sigmoid is exactly 1
+    float m40[4];               // 40 deg <111>
+};
+
 struct DomainArgs {
     DFront f[2];
     DevState* st;
@@ -1387,6 +1396,11 @@ __device__ __forceinline__ void d_grimmer(const DomainArgs& A, const double p[4]
     c[4][2] = __dmul_rn(__dadd_rn(__dadd_rn(__dsub_rn(a, b), cc), d), 0.5); c[4][3] = __dmul_rn(__dsub_rn(__dsub_rn(__dsub_rn(a, b), cc), d), 0.5);
     c[5][0] = a; c[5][1] = b; c[5][2] = cc; c[5][3] = d;
 }
+// |x| > m for m >= 0 by integers (the FP64 pipe runs at 1/64 rate); a NaN is not above anything
+__device__ __forceinline__ bool abs_above(double x, double m) {
+    const long long b = __double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll;
+    return b > __double_as_longlong(m) && b <= 0x7FF0000000000000ll;
+}
 // disorientation angle; `exact_zero` when the host also returns exactly 0
 __device__ __forceinline__ double d_disori(const DomainArgs& A, const double p[4], const double q[4], int* mi_out) {
     double c[6][4];
@@ -1397,11 +1411,88 @@ __device__ __forceinline__ double d_disori(const DomainArgs& A, const double p[4
     for (int i = 0; i < 6; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (fabs(c[i][j]) > om) { om = fabs(c[i][j]); mi = i; }
+            if (abs_above(c[i][j], om)) { om = fabs(c[i][j]); mi = i; }
     if (mi_out) *mi_out = mi;
     if (om < (1.0 - 5.0e-16)) return 2.0 * acos(om);
     return 0.0;
 }
+// ---- constant weights by FP32 ----
+// Most pairs' weights are constants (-1 low angle, 0 away from 40 deg <111>, Rollett-Holm's saturated 1), and
+// FP32 tells which wherever the pair is clear of every threshold by more than its rounding: FP64 runs at
+// 1/64 of its rate here.  Errors: a component of the misorientation is off by at most 4 products of
+// factors rounded to 24 bits and 3 sums, below 7e-7; a candidate sums 2 (times sqrt(1/2)) or 4 (times 1/2)
+// of them, below 1.5e-6; the second product has factors off by that much, its candidates below 1.3e-5.
+// The margins are five times that.
+constexpr float kWeightEps = 8e-6f, kWeightEps2 = 7e-5f;
+constexpr int kWeightUnknown = 2;
+
+// the largest component of each of the six symmetry families of (a, b, c, d), as d_grimmer orders them
+__device__ __forceinline__ void family_max(const float r[4], float f[6]) {
+    const float a = fabsf(r[0]), b = fabsf(r[1]), c = fabsf(r[2]), d = fabsf(r[3]);
+    const float s1 = fabsf(r[0] + r[1]), d1 = fabsf(r[0] - r[1]), s2 = fabsf(r[2] + r[3]), d2 = fabsf(r[2] - r[3]);
+    f[0] = fmaxf(a + b, c + d) * 0.70710678f;
+    f[1] = fmaxf(a + c, b + d) * 0.70710678f;
+    f[2] = fmaxf(a + d, b + c) * 0.70710678f;
+    f[3] = fmaxf(s1 + s2, d1 + d2) * 0.5f;
+    f[4] = fmaxf(s1 + d2, d1 + s2) * 0.5f;
+    f[5] = fmaxf(fmaxf(a, b), fmaxf(c, d));
+}
+// conj(q) p
+__device__ __forceinline__ void misorientation(const float p[4], const float q[4], float r[4]) {
+    r[0] = q[0] * p[0] + q[1] * p[1] + q[2] * p[2] + q[3] * p[3];
+    r[1] = p[1] * q[0] - p[0] * q[1] - q[2] * p[3] + q[3] * p[2];
+    r[2] = p[2] * q[0] - p[0] * q[2] + q[1] * p[3] - q[3] * p[1];
+    r[3] = p[3] * q[0] - p[0] * q[3] - q[1] * p[2] + q[2] * p[1];
+}
+// -1, 0 or 1: the weight is that constant; kWeightUnknown: too close to a threshold, or not a constant
+__device__ __noinline__ int weight_class(const WeightClass& w, float4 rx, float4 df) {
+    const float p[4] = {rx.x, rx.y, rx.z, rx.w}, q[4] = {df.x, df.y, df.z, df.w};
+    float r[4], f[6];
+    misorientation(p, q, r);
+    const float n2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+    if (!(fabsf(n2 - 1.0f) < 1e-3f)) return kWeightUnknown;  // the margins are for unit quaternions
+    family_max(r, f);
+    float om = f[0], om2 = -1.0f;  // largest, and the largest of another family
+    int mi = 0;
+#pragma unroll
+    for (int i = 1; i < 6; ++i) {
+        if (f[i] > om) { om2 = om; om = f[i]; mi = i; }
+        else om2 = fmaxf(om2, f[i]);
+    }
+    if (w.model == 2) return om < w.cos_sat - kWeightEps ? 1 : kWeightUnknown;
+    if (w.model != 1) return kWeightUnknown;
+    if (om > w.cos_lagb + kWeightEps) return -1;
+    if (!(om < w.cos_lagb - kWeightEps)) return kWeightUnknown;
+    // the deviation from 40 deg <111> is at least the difference of the angles
+    if (om > w.cos_lo + kWeightEps || om < w.cos_hi - kWeightEps) return 0;
+    if (!(om - om2 > 2.0f * kWeightEps)) return kWeightUnknown;  // the best candidate could be another one
+    float s[4];
+    if (mi == 5) {
+        s[0] = r[0]; s[1] = r[1]; s[2] = r[2]; s[3] = r[3];
+    } else if (mi >= 3) {
+        const float s1 = r[0] + r[1], d1 = r[0] - r[1], s2 = r[2] + r[3], d2 = r[2] - r[3];
+        const float u = mi == 3 ? s2 : d2, v = mi == 3 ? d2 : s2;
+        s[0] = 0.5f * (s1 + u); s[1] = 0.5f * (s1 - u); s[2] = 0.5f * (d1 + v); s[3] = 0.5f * (d1 - v);
+    } else {
+        const float b = mi == 0 ? r[1] : mi == 1 ? r[2] : r[3], c = mi == 0 ? r[2] : r[1], d = mi == 2 ? r[2] : r[3];
+        s[0] = (r[0] + b) * 0.70710678f; s[1] = (r[0] - b) * 0.70710678f;
+        s[2] = (c + d) * 0.70710678f; s[3] = (c - d) * 0.70710678f;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[i] = fabsf(s[i]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int k = 0; k < 3 - i; ++k) {
+            const float hi = fmaxf(s[k], s[k + 1]), lo = fminf(s[k], s[k + 1]);
+            s[k] = hi; s[k + 1] = lo;
+        }
+    misorientation(s, w.m40, r);
+    family_max(r, f);
+    const float dev = fmaxf(fmaxf(fmaxf(f[0], f[1]), fmaxf(f[2], f[3])), fmaxf(f[4], f[5]));
+    return dev < w.cos_dev - kWeightEps2 ? 0 : kWeightUnknown;
+}
+
 // P of a new cell from the table.  An unknown entry is requested from the host (FP64,
 // libm, on its worker threads): the first requester takes miss slot m (atomicAdd) and
 // tags the entry kPtabTag | m; every cell of the pair carries m and gets P from the host's
