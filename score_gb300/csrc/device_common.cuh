@@ -31,7 +31,8 @@ struct DevState {
     uint32_t next_never[2];     // slots ever used per list (Inside, Border)
     uint32_t err;               // sticky error flags
     uint32_t err_info;
-    uint32_t reserved[4];
+    uint32_t ntouch;            // P-table entries the device settled itself since the reset (DomainArgs::touched)
+    uint32_t reserved[3];
     // ---- per step ----
     uint32_t nfull[2];          // FullRX list lengths
     uint32_t ninactive[2];      // INACTIVE slots seen by the scan (uncapped)
@@ -41,6 +42,7 @@ struct DevState {
     uint32_t ntagged;           // new cells whose P waits for the host (tagged)
     uint32_t ndepleted;         // deformed grains whose last cell recrystallized
     uint32_t nnuc;              // nuclei placed on the device before this step's grow
+    uint32_t nknown;            // (rxg,defg) pairs met first whose constant weight the device settled
     uint32_t commit_done;       // commit blocks finished (the last one closes the step)
     unsigned long long sv[2];   // ACTIVE slots updated
     unsigned long long pmax_bits;  // max over new non-negative P (ordered bits)

@@ -629,13 +629,15 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
                 v.next_never[0] = n0; v.next_never[1] = n1;
                 v.err = __ldcg(&st->err) | (over_cap ? kErrCapacity : 0u);
                 v.err_info = 0;
-                for (int j = 0; j < 4; ++j) v.reserved[j] = 0;
+                v.ntouch = __ldcg(&st->ntouch);
+                for (int j = 0; j < 3; ++j) v.reserved[j] = 0;
                 v.nfull[0] = F0; v.nfull[1] = Ftot - F0;
                 v.ninactive[0] = I0; v.ninactive[1] = I1;
                 v.nrec[0] = nrec0; v.nrec[1] = nrec1;
                 v.nwin[0] = W0; v.nwin[1] = W1;
                 v.nmiss = __ldcg(&st->nmiss); v.ntagged = __ldcg(&st->ntagged);
                 v.ndepleted = __ldcg(&st->ndepleted); v.nnuc = __ldcg(&st->nnuc);
+                v.nknown = __ldcg(&st->nknown);
                 v.commit_done = 0;
                 v.sv[0] = p0 - I0; v.sv[1] = p1 - I1;
                 v.pmax_bits = __ldcg(&st->pmax_bits);
@@ -643,7 +645,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
                 box->snap = v;
                 st->next_never[0] = n0; st->next_never[1] = n1;
                 st->err = v.err;
-                st->nmiss = 0; st->ntagged = 0; st->ndepleted = 0; st->nnuc = 0; st->pmax_bits = 0;
+                st->nmiss = 0; st->ntagged = 0; st->nknown = 0; st->ndepleted = 0; st->nnuc = 0; st->pmax_bits = 0;
                 const uint32_t t_c = now_ns();
                 fh->phase_ns[0] = t_a - t_start; fh->phase_ns[1] = t_b - t_a; fh->phase_ns[2] = t_c - t_b; fh->phase_ns[3] = t_c - t_start;
                 if (w & kCmdLast) fd->bar = 0u;

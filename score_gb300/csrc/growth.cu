@@ -477,6 +477,7 @@ struct score_ctx {
     // P-table entries the runs since the last reset wrote (requests, nuclei): a reset clears these
     // instead of the whole table, unless the table is fresh or was loaded from the caller
     std::vector<unsigned long long> ptab_touched;
+    uint32_t ntouch = 0;               // entries the device settled itself (a.touched)
     bool ptab_dirty_all = true;
 
     ~score_ctx() { release_domain(); release_stream(); }
@@ -499,7 +500,7 @@ struct score_ctx {
 
 void score_ctx::release_domain() {
     if (device >= 0) cudaSetDevice(device);
-    void* ptrs[] = {a.fuse, a.f[0].inc, a.f[1].inc, scratch.inc, a.f[0].mob, a.f[1].mob, scratch.mob, a.f[0].fill, a.f[0].comp, a.f[0].vel, a.f[0].defg, a.f[0].rxg, a.f[0].xyz, a.f[0].dir, a.f[0].full, a.f[0].recyc,
+    void* ptrs[] = {a.fuse, a.touched, (void*)a.rxq, (void*)a.dfq, a.f[0].inc, a.f[1].inc, scratch.inc, a.f[0].mob, a.f[1].mob, scratch.mob, a.f[0].fill, a.f[0].comp, a.f[0].vel, a.f[0].defg, a.f[0].rxg, a.f[0].xyz, a.f[0].dir, a.f[0].full, a.f[0].recyc,
                     a.f[1].fill, a.f[1].comp, a.f[1].vel, a.f[1].defg, a.f[1].rxg, a.f[1].xyz, a.f[1].dir, a.f[1].full, a.f[1].recyc,
                     a.grid, a.claim, a.amask, a.ptab, a.defg_cnt, a.rxg_cnt, a.depleted, a.miss, a.tobm, a.ctcnt, a.fcell,
                     a.f[0].fmask, a.f[0].imask, a.f[0].tcnt, a.f[1].fmask, a.f[1].imask, a.f[1].tcnt,
@@ -1073,10 +1074,17 @@ int reset_state(score_ctx* c) {
         // entries the last runs wrote (a 512^3 run writes about 0.03 % of its 8 GB table)
         const size_t total = std::max<size_t>((size_t)c->nrxg * c->ndefg, 1);
         const size_t nt = c->ptab_touched.size();
-        if (c->failed) c->ptab_dirty_all = true;  // a step that failed may have tagged entries it never reported
-        if (c->ptab_dirty_all || nt > total / 64 || !c->stage(nt * 8)) {
+        if (c->failed || c->ntouch > a.touchcap) c->ptab_dirty_all = true;  // a step that failed may have tagged entries it never reported
+        if (c->ptab_dirty_all || nt + c->ntouch > total / 64 || !c->stage(nt * 8)) {
             e = cudaMemsetAsync(a.ptab, 0xFF, total * 8, st);
-        } else if (nt) {
+        } else {
+            if (c->ntouch) {
+                k_clear_ptab<<<blocks_for(c->ntouch, c->sms), kBlock, 0, st>>>(a.ptab, a.touched, c->ntouch);
+                c->launches++;
+                e = cudaGetLastError();
+            }
+        }
+        if (e == cudaSuccess && nt && !(c->ptab_dirty_all || nt + c->ntouch > total / 64)) {
             e = cudaMemcpyAsync(c->d_stage, c->ptab_touched.data(), nt * 8, cudaMemcpyHostToDevice, st);
             if (e == cudaSuccess) {
                 k_clear_ptab<<<blocks_for(nt, c->sms), kBlock, 0, st>>>(a.ptab, (const unsigned long long*)c->d_stage, (uint32_t)nt);
@@ -1085,6 +1093,7 @@ int reset_state(score_ctx* c) {
             }
         }
         c->ptab_touched.clear();
+        c->ntouch = 0;
         c->ptab_dirty_all = false;
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(a.defg_cnt, c->d_defg_cnt_init, (size_t)c->ndefg * 4, cudaMemcpyDeviceToDevice, st);
@@ -1265,6 +1274,7 @@ int post_step(score_ctx* c, uint32_t newnuc, score_step_stats* out) {
     double pmax_new = 0.0;
     if (hs.pmax_bits) memcpy(&pmax_new, &hs.pmax_bits, 8);
     uint32_t nreq = 0;  // distinct weights requested (void race slots excluded)
+    c->ntouch = hs.ntouch;
     if (c->ans_ready) {  // computed by the engine over all domains' requests
         c->ans_ready = false;
         for (double v : c->ans_val) if (v > pmax_new) pmax_new = v;
@@ -1357,7 +1367,7 @@ int post_step(score_ctx* c, uint32_t newnuc, score_step_stats* out) {
     o.Pmax = ph.Pmax; o.rhomax = rhomax_step; o.dXstep = 0.0;
     o.next_never[0] = c->next_never[0]; o.next_never[1] = c->next_never[1];
     o.n_recycled[0] = hs.nrec[0]; o.n_recycled[1] = hs.nrec[1];
-    o.p_misses = nreq;
+    o.p_misses = nreq + hs.nknown;  // pairs met first in this step
     if (out) *out = o;
     return SCORE_OK;
 }
@@ -2402,6 +2412,10 @@ int score_load_domain(score_ctx* c, const uint32_t* grid, const double* defg_qua
         if (e == cudaSuccess) e = dalloc(&a.rxg_cnt, nrxg);
         if (e == cudaSuccess) e = dalloc(&a.depleted, ndefg);
         if (e == cudaSuccess) e = dalloc(&a.miss, a.misscap);
+        a.touchcap = std::min<uint32_t>(a.misscap, 1u << 22);
+        if (e == cudaSuccess) e = dalloc(&a.touched, a.touchcap);
+        if (e == cudaSuccess) e = dalloc((float4**)&a.rxq, nrxg);
+        if (e == cudaSuccess) e = dalloc((float4**)&a.dfq, ndefg);
         if (e == cudaSuccess) e = dalloc(&c->d_state, 1);
         if (e == cudaSuccess) e = dalloc(&a.fuse, 1);
         if (e == cudaSuccess) e = cudaMemsetAsync(a.fuse, 0, sizeof(FuseDom), c->stream);
@@ -2422,6 +2436,15 @@ int score_load_domain(score_ctx* c, const uint32_t* grid, const double* defg_qua
     } else {
         c->high_water[0] = std::max(c->high_water[0], c->next_never[0]);
         c->high_water[1] = std::max(c->high_water[1], c->next_never[1]);
+    }
+    {   // orientations in FP32 for the classification of new pairs (none where the caller gave every weight)
+        std::vector<float> q(4 * ((size_t)nrxg + ndefg));
+        for (size_t i = 0; i < 4 * (size_t)nrxg; ++i) q[i] = (float)rxg_quat[i];
+        for (size_t i = 0; i < 4 * (size_t)ndefg; ++i) q[4 * (size_t)nrxg + i] = (float)defg_quat[i];
+        if (nrxg) e = cudaMemcpyAsync((void*)a.rxq, q.data(), (size_t)nrxg * 16, cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync((void*)a.dfq, q.data() + 4 * (size_t)nrxg, (size_t)ndefg * 16, cudaMemcpyHostToDevice, c->stream);
+        if (e != cudaSuccess) return c->cuda_fail(e, "load domain");
+        a.cls = make_weight_class(p);
     }
     // the linear grid goes through the claim array (reset before the first step) into bricks
     e = cudaMemcpyAsync(a.claim, grid, N * 4, cudaMemcpyHostToDevice, c->stream);

@@ -129,6 +129,11 @@ struct DomainArgs {
     float dtc32;
     int32_t spec;               // few INACTIVE slots last step: k_grow_fill loads every slot's data with its
                                 // infector byte instead of only the ACTIVE slots' (no effect on results)
+    const float4* rxq;          // orientations in FP32, for the classification of new pairs
+    const float4* dfq;
+    unsigned long long* touched;   // P-table entries the device settled itself (a reset clears these)
+    uint32_t touchcap;
+    WeightClass cls;
     double pc_fac;              // 1/sqrt(2) as the host computes it (the disorientation of d_grimmer)
 };
 
@@ -1493,21 +1498,31 @@ __device__ __noinline__ int weight_class(const WeightClass& w, float4 rx, float4
     return dev < w.cos_dev - kWeightEps2 ? 0 : kWeightUnknown;
 }
 
-// P of a new cell from the table.  An unknown entry is requested from the host (FP64,
-// libm, on its worker threads): the first requester takes miss slot m (atomicAdd) and
-// tags the entry kPtabTag | m; every cell of the pair carries m and gets P from the host's
-// answer m in the next step's k_grow_fill.  A requester that loses the race to tag the
-// entry voids its slot.  Returns true with P, or false with the tag.  (Classifying the
-// exact-constant weights on the device cost more than it saved: FP64 runs at 1/64 rate,
-// cells racing on a new pair all classify it, and the classifier's registers took a
-// quarter of this kernel's occupancy.)
+// P of a new cell from the table.  An unknown entry whose weight FP32 shows to be one of the constants gets
+// it here (94 % of random pairs: 0.3 M of a 512^3 run's pairs no longer travel to the host and back, and most
+// steps of small domains ask the host nothing).  The rest is requested from the host (FP64, libm, on its
+// worker threads): the first requester takes miss slot m (atomicAdd) and tags the entry kPtabTag | m; every
+// cell of the pair carries m and gets P from the host's answer m in the next step's fill.  A requester that
+// loses the race to tag the entry voids its slot.  Returns true with P, or false with the tag.  (Classifying
+// in FP64 cost more than it saved: 1/64 rate, and its registers took a quarter of the commit's occupancy;
+// weight_class is a call on the rare path.)
 __device__ __forceinline__ bool lookup_p(const DomainArgs& a, uint32_t rxg, uint32_t defg, double& P, uint32_t& tag) {
     const unsigned long long idx = (unsigned long long)rxg * a.ndefg + defg;
     unsigned long long* e = &a.ptab[idx];
-    // a plain (L1-cached) load: within a launch an entry only goes from EMPTY to a tag, and a stale
-    // EMPTY is settled by the compare-and-swap below
+    // a plain (L1-cached) load: within a launch phase an entry only goes from EMPTY to a tag or a constant, and
+    // a stale EMPTY is settled by the compare-and-swap below
     unsigned long long bits = *e;
     if (bits == kPtabEmpty) {
+        const int c = weight_class(a.cls, a.rxq[rxg], a.dfq[defg]);
+        if (c != kWeightUnknown) {
+            P = __hiloint2double(c == 0 ? 0 : c < 0 ? (int)0xBFF00000u : 0x3FF00000, 0);
+            if (atomicCAS(e, kPtabEmpty, (unsigned long long)__double_as_longlong(P)) == kPtabEmpty) {
+                const uint32_t q = atomicAdd(&a.st->ntouch, 1u);
+                if (q < a.touchcap) a.touched[q] = idx;
+                atomicAdd(&a.st->nknown, 1u);
+            }
+            return true;
+        }
         const uint32_t m = atomicAdd(&a.st->nmiss, 1u);
         if (m >= a.misscap) { atomicOr(&a.st->err, kErrMissCap); tag = 0; return false; }
         const unsigned long long old = atomicCAS(e, kPtabEmpty, kPtabTag | m);
