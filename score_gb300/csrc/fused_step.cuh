@@ -128,6 +128,11 @@ __device__ __forceinline__ bool group_barrier(FuseShared& sh, uint32_t* bar, uin
     return sh.ok != 0u;
 }
 
+// a wait that gave up: where (1 to 4 the step's barriers, 5 the host's word), the block, and how far it was
+__device__ __forceinline__ void fuse_gave_up(DevState* st, uint32_t where, uint32_t rank, uint32_t at) {
+    if (atomicCAS(&st->err_info, 0u, (where << 28) | ((rank & 0xFFFu) << 16) | (at & 0xFFFFu)) == 0u) atomicOr(&st->err, kErrTimeout);
+}
+
 // Block-wide inclusive scan of (x, y); the block's totals in tx, ty.  The caller's values come back exclusive.
 __device__ __forceinline__ void block_scan2(FuseShared& sh, uint32_t& x, uint32_t& y, uint32_t& tx, uint32_t& ty) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -301,7 +306,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
                     w = ld_relaxed_gpu(&fd->go);
                     ok = (w >> kCmdShift) == seq;
                 }
-                if (!ok) { atomicOr(&st->err, kErrTimeout); w = kCmdLeave; }
+                if (!ok) { fuse_gave_up(st, 5u, rank, seq); w = kCmdLeave; }
                 fence_gpu();
                 sh.word = w;
             }
@@ -326,7 +331,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             const double* src = fd->pay.pf_src;
             for (uint32_t g = rank * kFuse + threadIdx.x; g < a.ndefg; g += G * kFuse) ((double*)a.pforce)[g] = src[g];
             arrived += G;
-            if (!group_barrier(sh, &fd->bar, G, arrived, true)) { if (threadIdx.x == 0) atomicOr(&st->err, kErrTimeout); return; }
+            if (!group_barrier(sh, &fd->bar, G, arrived, true)) { if (threadIdx.x == 0) fuse_gave_up(st, 1u, rank, arrived); return; }
         }
         __syncthreads();
 
@@ -426,7 +431,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             }
         }
         arrived += G;
-        if (!group_barrier(sh, &fd->bar, G, arrived, true)) { if (threadIdx.x == 0) atomicOr(&st->err, kErrTimeout); return; }
+        if (!group_barrier(sh, &fd->bar, G, arrived, true)) { if (threadIdx.x == 0) fuse_gave_up(st, 2u, rank, arrived); return; }
         const uint32_t t_a = now_ns();
 
         // ---- B: recycle list, wins
@@ -503,7 +508,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
         __syncthreads();
         for (uint32_t lt = threadIdx.x; lt < nlt; lt += kFuse) cntB[rank + lt * G] = make_uint2(sh.tw[0][lt], sh.tw[1][lt]);
         arrived += G;
-        if (!group_barrier(sh, &fd->bar, G, arrived, true)) { if (threadIdx.x == 0) atomicOr(&st->err, kErrTimeout); return; }
+        if (!group_barrier(sh, &fd->bar, G, arrived, true)) { if (threadIdx.x == 0) fuse_gave_up(st, 3u, rank, arrived); return; }
         const uint32_t t_b = now_ns();
 
         // ---- C: commit
@@ -609,7 +614,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
         }
         if (__any_sync(0xFFFFFFFFu, pmax > 0.0 || ntag)) flush_new(a, pmax, ntag);
         arrived += G;
-        if (!group_barrier(sh, &fd->bar, G, arrived, first)) { if (threadIdx.x == 0) atomicOr(&st->err, kErrTimeout); return; }
+        if (!group_barrier(sh, &fd->bar, G, arrived, first)) { if (threadIdx.x == 0) fuse_gave_up(st, 4u, rank, arrived); return; }
         // the lists' ends after this step, the same in every block
         const uint32_t p0 = n0, p1 = n1;
         if (W0 > nrec0) n0 += W0 - nrec0;
@@ -628,7 +633,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
                 DevState v;
                 v.next_never[0] = n0; v.next_never[1] = n1;
                 v.err = __ldcg(&st->err) | (over_cap ? kErrCapacity : 0u);
-                v.err_info = 0;
+                v.err_info = __ldcg(&st->err_info);
                 v.ntouch = __ldcg(&st->ntouch);
                 for (int j = 0; j < 3; ++j) v.reserved[j] = 0;
                 v.nfull[0] = F0; v.nfull[1] = Ftot - F0;

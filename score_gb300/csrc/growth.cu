@@ -883,7 +883,9 @@ void resolve_weights(score_ctx* c, const std::vector<unsigned long long>& idx, s
 
 int check_device_errors(score_ctx* c, uint32_t flags) {
     if (!flags) return SCORE_OK;
-    if (flags & kErrTimeout) return c->fail(SCORE_ERR_TIMEOUT, "a bounded device wait gave up (look-back scan)");
+    if (flags & kErrTimeout)
+        return c->fail(SCORE_ERR_TIMEOUT, "a bounded device wait gave up (at " + std::to_string(c->h_box->snap.err_info >> 28) + ", block " +
+                                              std::to_string((c->h_box->snap.err_info >> 16) & 0xFFFu) + ")");
     if (flags & kErrKeyLimit) return c->fail(SCORE_ERR_KEYLIMIT, "more than 2^32-1 infection attempts in one step");
     if (flags & kErrBorderRef) return c->fail(SCORE_ERR_BORDER_CAPACITY, "Border list exceeded 2(xy+xz+yz) slots (the reference writes out of bounds here)");
     if (flags & kErrCapacity) return c->fail(SCORE_ERR_CAPACITY, "front list capacity exceeded");
@@ -2075,7 +2077,10 @@ int make_ctx(const score_params* p, Engine* eng, bool own, score_ctx** out) {
         delete c;
         return SCORE_ERR_CUDA;
     }
-    memset(c->h_box, 0, sizeof(DevState));
+    // pinned memory comes back from an earlier context as that one left it: a post or a notice of leaving
+    // with the number of a step of this context would be taken for its own
+    memset(&c->h_box->fuse, 0, sizeof(FuseHost));
+    memset(&c->h_box->snap, 0, sizeof(DevState));
     *out = c;
     return SCORE_OK;
 }

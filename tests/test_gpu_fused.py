@@ -107,3 +107,25 @@ def test_batch_groups(gpu, tmp_path, ndom):
         b.run_until()
         for i, k in enumerate(pick):
             assert_same(first[i] + b.trace(i), b.labels(i), *b.grain_counts(i), refs[k])
+
+
+def test_contexts_one_after_another(gpu, tmp_path):
+    """A new context's mailbox may be the pinned memory of one that has gone: nothing in it counts."""
+    short, long = make("one_tile", tmp_path), make("odd_periodic", tmp_path)
+    refs = [oracle.run(p, d) for p, d in (short, long)]
+    assert len(refs[0]["trace"]) < len(refs[1]["trace"])
+    for _ in range(3):
+        for (p, d), ref in zip((short, long), refs):
+            with sg.GrowthMachine(p) as gm:
+                gm.load_domain(d)
+                gm.place_nuclei()
+                tr = gm.run_until()
+                assert_same(tr, gm.labels(), *gm.grain_counts(), ref)
+        pick = [short, long, short, long]
+        with sg.Batch([p for p, _ in pick]) as b:
+            for i, (_, d) in enumerate(pick):
+                b.load_domain(i, d)
+            b.place_nuclei()
+            b.run_until()
+            for i in range(4):
+                assert_same(b.trace(i), b.labels(i), *b.grain_counts(i), refs[i % 2])
