@@ -3,10 +3,10 @@
 // What bounds such a domain is neither bytes nor operations but the chain of a step: five or six
 // launches, each with its own start, constant-cache misses and dependent loads, then a stream
 // synchronization and the host's master block (64^3 domain, front of 30 k slots: 51 us a step, of which the
-// bytes take 0.1; 128^3: 59 us; here 26 and 33).  A group of blocks steps one domain inside one
+// bytes take 0.1; 128^3: 59 us; here 25 and 28).  A group of blocks steps one domain inside one
 // cooperative launch:
-//   A  fill of the group's tiles; full cells into records; the 26 infection attempts of every full
-//      cell, a warp per full cell and a lane per direction.  The attempt ordinal is 26 s + d with s the
+//   A  fill of the group's tiles, 2 or 4 consecutive slots a thread; full cells into records; the 26 infection
+//      attempts of every full cell, four lanes a cell.  The attempt ordinal is 26 s + d with s the
 //      full cell's slot (Border slots after the Inside ones) instead of its rank among the full cells:
 //      the same order, and no list has to exist before the claims;
 //   -- group barrier --
@@ -28,13 +28,18 @@ namespace score {
 constexpr int kFuse = 1024;                               // threads per block, one block per SM
 // 1,024 threads of 64 registers: 512 of 110 took 10 % more on the 64^3 domain and 24 % on a recovering 384^3 one
 constexpr int kFuseWarps = kFuse / 32;
-constexpr int kFuseItems = 2;
-constexpr uint32_t kFuseTile = kFuse * kFuseItems;        // slots per tile
-constexpr uint32_t kFuseTileWords = kFuseTile / 32;
-static_assert(kFuseTileWords == 32 * kFuseItems && kFuseWarps == 32, "a word of a tile per warp and item");
+// slots per tile: ITEMS per thread
+template <int ITEMS>
+struct FuseShape {
+    static constexpr uint32_t kTile = kFuse * ITEMS;
+    static constexpr uint32_t kWords = kTile / 32;
+    static_assert(kWords == 32 * ITEMS && kFuseWarps == 32, "a word of a tile per warp and item");
+};
 constexpr uint32_t kFuseMaxTiles = 4096;                  // tiles of a domain (both lists)
 constexpr uint32_t kFuseMaxLocal = 512;                   // tiles of one block
-constexpr uint32_t kFuseRec = 3072;                       // full cells of a block and step kept in shared memory
+constexpr uint32_t kFuseRec = 2048;                       // full cells of a block and step kept in shared memory
+constexpr uint32_t kFuseMask = 2048;                      // mask words of a block kept in shared memory
+constexpr uint32_t kFuseWins = 4096;                      // new cells listed at a time
 constexpr uint32_t kFuseSpin = 1u << 22;                  // polls of a group wait before it gives up (seconds)
 constexpr uint32_t kFuseHostSpin = 1u << 12;              // polls of the host's answer before the group leaves (milliseconds)
 
@@ -99,8 +104,8 @@ struct FuseShared {
     uint32_t rec_win[kFuseRec];        // attempts made, then attempts won
     uint32_t rec_tob[kFuseRec];        // won attempts that go to the Border list
     uint16_t rec_lt[kFuseRec];         // the record's tile among the block's
-    uint32_t fm[kFuse], im[kFuse];     // full and INACTIVE masks of the block's tiles while they fit
-    uint16_t wl[kFuse * 26];           // wins of a chunk of records: record in the chunk << 5 | direction
+    uint32_t fm[kFuseMask], im[kFuseMask];         // full and INACTIVE masks of the block's tiles while they fit
+    uint16_t wl[kFuseWins];            // new cells of a chunk of records: record in the chunk << 5 | direction
     uint32_t c_win[kFuse], c_tob[kFuse], c_rA[kFuse], c_rB[kFuse], c_cell[kFuse], c_rs[kFuse];
     double c_over[kFuse];
     uint32_t tw[2][kFuseMaxLocal];     // wins of the block's tiles per destination list
@@ -108,6 +113,7 @@ struct FuseShared {
     uint32_t off[kFuseMaxLocal + 1];   // first record of each of the block's tiles
     uint32_t w1[kFuseWarps], w2[kFuseWarps], w3[kFuseWarps];
     uint32_t t0[2], tot[2];            // counts before the Border list's tiles, and in all
+    uint32_t dir[26];                  // directions for moore_word
     uint32_t word, ok;
 };
 
@@ -189,41 +195,74 @@ __device__ __forceinline__ void tile_scan(FuseShared& sh, const uint2* cnt, uint
     __syncthreads();
 }
 
-// target_of for a lane's own direction
-__device__ __forceinline__ bool target_lane(const DomainArgs& a, int L, int x, int y, int z, int dx, int dy, int dz, uint32_t& t,
-                                            bool& interior) {
-    int tx = x + dx, ty = y + dy, tz = z + dz;
-    if (L == 1) {
-        if (tx < 0) tx += (int)a.nx;
-        if (tx >= (int)a.nx) tx -= (int)a.nx;
-        if (ty < 0) ty += (int)a.ny;
-        if (ty >= (int)a.ny) ty -= (int)a.ny;
-        if (a.boundary == 0) {
-            if (tz < 0 || tz >= (int)a.nz) return false;
-        } else {
-            if (tz < 0) tz += (int)a.nz;
-            if (tz >= (int)a.nz) tz -= (int)a.nz;
-        }
-    } else if (tx < 0 || ty < 0 || tz < 0 || tx >= (int)a.nx || ty >= (int)a.ny || tz >= (int)a.nz) {
+// The grid words of a cell's 26 neighbours as sums of three terms: in bricks, a word is
+// 8 ((z/2) gbxy + (y/2) gbx + x/2) + 4 (z%2) + 2 (y%2) + x%2, so each axis gives a term for -1, 0 and +1 with its
+// wrap done once.  Border cells wrap in x and y and drop z (reference) or wrap it (periodic option); Inside
+// cells are strictly interior.
+struct Moore {
+    uint32_t X[3], Y[3], Z[3];
+    uint32_t open;     // bit k: offset k - 1 along z exists
+    uint32_t inner;    // bits 0-2 x, 3-5 y, 6-8 z: the offset's coordinate is not on a face
+    bool near;         // the cell lies on the second layer below a face: an Inside cell's infections go to the Border list
+};
+__device__ __forceinline__ bool moore_of(const DomainArgs& a, int L, uint32_t cell, Moore& m) {
+    int x, y, z;
+    decode(a, cell, x, y, z);
+    const int nx = (int)a.nx, ny = (int)a.ny, nz = (int)a.nz;
+    if (L == 0 && !(x > 0 && y > 0 && z > 0 && x < nx - 1 && y < ny - 1 && z < nz - 1)) {
         atomicOr(&a.st->err, kErrBounds);
         return false;
     }
-    interior = tx > 0 && tx < (int)a.nx - 1 && ty > 0 && ty < (int)a.ny - 1 && tz > 0 && tz < (int)a.nz - 1;
-    t = gindex(a, (uint32_t)tx, (uint32_t)ty, (uint32_t)tz);
+    m.open = 0u; m.inner = 0u;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        int tx = x + k - 1, ty = y + k - 1, tz = z + k - 1;
+        if (tx < 0) tx += nx;
+        if (tx >= nx) tx -= nx;
+        if (ty < 0) ty += ny;
+        if (ty >= ny) ty -= ny;
+        bool in = true;
+        if (tz < 0) { in = a.boundary != 0; tz += nz; }
+        if (tz >= nz) { in = a.boundary != 0; tz -= nz; }
+        m.X[k] = (((uint32_t)tx >> 1) << 3) | ((uint32_t)tx & 1u);
+        m.Y[k] = ((((uint32_t)ty >> 1) * a.gbx) << 3) | (((uint32_t)ty & 1u) << 1);
+        m.Z[k] = ((((uint32_t)tz >> 1) * a.gbxy) << 3) | (((uint32_t)tz & 1u) << 2);
+        m.open |= (in ? 1u : 0u) << k;
+        m.inner |= (tx > 0 && tx < nx - 1 ? 1u : 0u) << k;
+        m.inner |= (ty > 0 && ty < ny - 1 ? 8u : 0u) << k;
+        m.inner |= (tz > 0 && tz < nz - 1 ? 64u : 0u) << k;
+    }
+    m.near = !(x > 1 && x < nx - 2 && y > 1 && y < ny - 2 && z > 1 && z < nz - 2);
     return true;
+}
+// the neighbour in a direction packed as (dx + 1) | (dy + 1) << 2 | (dz + 1) << 4; false where z is open
+__device__ __forceinline__ bool moore_word(const Moore& m, uint32_t dir, uint32_t& t, bool& interior) {
+    const uint32_t i = dir & 3u, j = (dir >> 2) & 3u, k = dir >> 4;
+    t = (i == 0 ? m.X[0] : i == 1 ? m.X[1] : m.X[2]) + (j == 0 ? m.Y[0] : j == 1 ? m.Y[1] : m.Y[2]) + (k == 0 ? m.Z[0] : k == 1 ? m.Z[1] : m.Z[2]);
+    interior = ((m.inner >> i) & (m.inner >> (3u + j)) & (m.inner >> (6u + k)) & 1u) != 0u;
+    return (m.open >> k) & 1u;
+}
+
+// overshoot of a full cell, for the cells it infects
+template <bool FP32>
+__device__ __forceinline__ double full_over(const DFront& fr, uint32_t slot) {
+    if (!FP32) return __dsub_rn(((const double*)fr.fill)[slot], 1.0);
+    return (double)((((const float*)fr.fill)[slot] - 1.0f) - fr.comp[slot]);
 }
 
 // The records of a block's full cells: the first kFuseRec in shared memory, the rest in the domain's per-full-cell
 // arrays at the full cell's own slot position (a position no other full cell has; n0 + n1 slots never exceed the
 // arrays' N words, as every slot stands for a cell infected once).  `pos` is looked up from the tile offsets.
+template <int ITEMS>
 struct FuseRecs {
+    static constexpr uint32_t kTile = FuseShape<ITEMS>::kTile;
     FuseShared& sh;
     uint32_t rank, G, T0, n0, nlt;
     __device__ __forceinline__ uint32_t pos(uint32_t i) const {
         uint32_t lt = nlt - 1;
         while (sh.off[lt] > i) --lt;
         const uint32_t u = rank + lt * G;
-        return (u >= T0 ? n0 + (u - T0) * kFuseTile : u * kFuseTile) + (i - sh.off[lt]);
+        return (u >= T0 ? n0 + (u - T0) * kTile : u * kTile) + (i - sh.off[lt]);
     }
     __device__ __forceinline__ uint32_t key(uint32_t i) const { return i < kFuseRec ? sh.rec_key[i] : sh.a.f[0].full[pos(i)]; }
     __device__ __forceinline__ uint32_t cell(uint32_t i) const { return i < kFuseRec ? sh.rec_cell[i] : sh.a.fcell[pos(i)]; }
@@ -236,20 +275,242 @@ struct FuseRecs {
     // local tile of record i with key k
     __device__ __forceinline__ uint32_t tile(uint32_t i, uint32_t k) const {
         if (i < kFuseRec) return sh.rec_lt[i];
-        const uint32_t tl = (k & 0x7FFFFFFFu) / kFuseTile;
+        const uint32_t tl = (k & 0x7FFFFFFFu) / kTile;
         return ((k >> 31 ? T0 + tl : tl) - rank) / G;
     }
 };
 
-template <bool FP32>
-__device__ __forceinline__ void fuse_grow(const DomainArgs& a, const DFront& fr, uint32_t base, uint32_t n, uint32_t& act, uint32_t& full) {
-    if (a.refresh == 2) grow_items<FP32, 2, kFuseItems>(a, fr, base, n, act, full);
-    else if (a.refresh == 1) grow_items<FP32, 1, kFuseItems>(a, fr, base, n, act, full);
-    else if (a.spec && !a.dt_changed) grow_items<FP32, 3, kFuseItems>(a, fr, base, n, act, full);
-    else grow_items<FP32, 0, kFuseItems>(a, fr, base, n, act, full);
+// V consecutive values as one access (4 or 2 of 1, 4 or 8 bytes; 32 bytes as two)
+template <int V> struct Vec;
+template <> struct Vec<2> {
+    static __device__ __forceinline__ uint32_t bytes(const uint8_t* p) { return *(const uint16_t*)p | 0xFFFF0000u; }
+    static __device__ __forceinline__ void load(const double* p, double (&v)[2]) { const double2 x = *(const double2*)p; v[0] = x.x; v[1] = x.y; }
+    static __device__ __forceinline__ void load(const float* p, float (&v)[2]) { const float2 x = *(const float2*)p; v[0] = x.x; v[1] = x.y; }
+    static __device__ __forceinline__ void load(const uint32_t* p, uint32_t (&v)[2]) { const uint2 x = *(const uint2*)p; v[0] = x.x; v[1] = x.y; }
+    static __device__ __forceinline__ void store(double* p, const double (&v)[2]) { *(double2*)p = make_double2(v[0], v[1]); }
+    static __device__ __forceinline__ void store(float* p, const float (&v)[2]) { *(float2*)p = make_float2(v[0], v[1]); }
+};
+template <> struct Vec<4> {
+    static __device__ __forceinline__ uint32_t bytes(const uint8_t* p) { return *(const uint32_t*)p; }
+    static __device__ __forceinline__ void load(const double* p, double (&v)[4]) {
+        const double2 x = *(const double2*)p, y = *(const double2*)(p + 2);
+        v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+    }
+    static __device__ __forceinline__ void load(const float* p, float (&v)[4]) { const float4 x = *(const float4*)p; v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
+    static __device__ __forceinline__ void load(const uint32_t* p, uint32_t (&v)[4]) { const uint4 x = *(const uint4*)p; v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
+    static __device__ __forceinline__ void store(double* p, const double (&v)[4]) { *(double2*)p = make_double2(v[0], v[1]); *(double2*)(p + 2) = make_double2(v[2], v[3]); }
+    static __device__ __forceinline__ void store(float* p, const float (&v)[4]) { *(float4*)p = make_float4(v[0], v[1], v[2], v[3]); }
+};
+
+// infector bytes of slots s .. s + V - 1 of a list of n slots (INACTIVE past the list)
+template <int V>
+__device__ __forceinline__ uint32_t fuse_dirs(const DFront& fr, uint32_t s, uint32_t n) {
+    if (s + V <= n) return Vec<V>::bytes(fr.dir + s);
+    uint32_t w = 0xFFFFFFFFu;
+    for (uint32_t k = 0; s + k < n; ++k) w = (w & ~(0xFFu << (8 * k))) | ((uint32_t)fr.dir[s + k] << (8 * k));
+    return w;
 }
 
-template <bool FP32>
+// The fill update of V consecutive slots with infector bytes dw, the arithmetic of grow_items.  V slots are one
+// access a field (slot V-aligned, arrays 256-byte aligned): whole sectors move in FP64 whether one of four
+// slots is ACTIVE or all, so a hole costs nothing but its byte unless the four are mixed, and the fields of
+// INACTIVE slots among them are written back as they were read (increments, velocities and mobilities of an
+// INACTIVE slot mean nothing).  act / full: bit k for slot s + k.
+template <bool FP32, int V>
+__device__ __forceinline__ void fuse_grow(const DomainArgs& a, const DFront& fr, uint32_t s, uint32_t dw, uint32_t& act, uint32_t& full) {
+    act = 0; full = 0;
+#pragma unroll
+    for (int k = 0; k < V; ++k)
+        if (((dw >> (8 * k)) & 0xFFu) != kInactive) act |= 1u << k;
+    if (!act) return;
+    const bool whole = s + V <= fr.cap;  // else the last slots of the list's arrays, one by one
+    using X = Vec<V>;
+    if (!FP32) {
+        double w[V], fill[V];
+        double* const pf = (double*)fr.fill + s;
+        double* const pv = (double*)fr.vel + s;
+        double* const pi = fr.inc + s;
+        if (whole) X::load((const double*)pf, fill);
+        else
+#pragma unroll
+            for (int k = 0; k < V; ++k) fill[k] = (act >> k) & 1u ? pf[k] : 0.0;
+        const bool dtc = a.dt_changed != 0;
+        if (a.refresh == 0) {
+            const double* src = dtc ? pv : pi;
+            if (whole) X::load(src, w);
+            else
+#pragma unroll
+                for (int k = 0; k < V; ++k) w[k] = (act >> k) & 1u ? src[k] : -1.0;
+#pragma unroll
+            for (int k = 0; k < V; ++k) {  // nuclei, cells answered by the host: no increment yet
+                const uint8_t d = (uint8_t)(dw >> (8 * k));
+                if (!((act >> k) & 1u) || !(d & kStale)) continue;
+                if (d & kPend) {
+                    w[k] = answered_velocity(a, fr, s + k, d, ((const unsigned long long*)fr.vel)[s + k]);
+                    pv[k] = w[k];
+                } else if (!dtc) {
+                    w[k] = pv[k];
+                }
+            }
+        } else {
+            double mo[V];
+            uint32_t g[V];
+            if (whole) X::load((const uint32_t*)fr.defg + s, g);
+            else
+#pragma unroll
+                for (int k = 0; k < V; ++k) g[k] = (act >> k) & 1u ? fr.defg[s + k] : 0u;
+            if (a.refresh == 2) {
+                if (whole) X::load((const double*)fr.mob + s, mo);
+                else
+#pragma unroll
+                    for (int k = 0; k < V; ++k) mo[k] = (act >> k) & 1u ? fr.mob[s + k] : 0.0;
+            } else {
+                uint32_t r[V];
+                if (whole) X::load((const uint32_t*)fr.rxg + s, r);
+                else
+#pragma unroll
+                    for (int k = 0; k < V; ++k) r[k] = (act >> k) & 1u ? fr.rxg[s + k] : 0u;
+#pragma unroll
+                for (int k = 0; k < V; ++k) {
+                    mo[k] = 0.0;
+                    if (((act >> k) & 1u) && !((dw >> (8 * k)) & kPend))
+                        mo[k] = mobility(a, __longlong_as_double((long long)a.ptab[(unsigned long long)r[k] * a.ndefg + g[k]]));
+                }
+                if (whole) X::store(fr.mob + s, mo);
+                else
+#pragma unroll
+                    for (int k = 0; k < V; ++k) if ((act >> k) & 1u) fr.mob[s + k] = mo[k];
+            }
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+                const uint8_t d = (uint8_t)(dw >> (8 * k));
+                w[k] = -1.0;
+                if (!((act >> k) & 1u)) continue;
+                if (d & kPend) w[k] = answered_velocity(a, fr, s + k, d, ((const unsigned long long*)fr.vel)[s + k]);
+                else w[k] = velocity_from_mobility(a, mo[k], g[k], d & kCodeMask);
+            }
+            if (whole) X::store(pv, w);
+            else
+#pragma unroll
+                for (int k = 0; k < V; ++k) if ((act >> k) & 1u) pv[k] = w[k];
+        }
+        const bool fresh = dtc || a.refresh != 0;  // every increment is new
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            const uint8_t d = (uint8_t)(dw >> (8 * k));
+            if (!((act >> k) & 1u)) { w[k] = -1.0; continue; }
+            if (fresh || (d & kStale)) {
+                if (__double_as_longlong(w[k]) >= 0) w[k] = __dmul_rn(__dmul_rn(w[k], a.dt), a.cinv);
+                if (!fresh) pi[k] = w[k];
+                if (d & kStale) fr.dir[s + k] = d & kCodeMask;
+            }
+        }
+        if (fresh) {
+            if (whole) X::store(pi, w);
+            else
+#pragma unroll
+                for (int k = 0; k < V; ++k) if ((act >> k) & 1u) pi[k] = w[k];
+        }
+        uint32_t moved = 0;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            if (__double_as_longlong(w[k]) < 0) continue;  // INACTIVE, or no driving force
+            fill[k] = __dadd_rn(fill[k], w[k]);
+            moved |= 1u << k;
+            if (__double_as_longlong(fill[k]) >= 0x3FF0000000000000ll) full |= 1u << k;  // f >= 1.0, never negative
+        }
+        if (whole) { if (moved) X::store(pf, fill); }
+        else
+#pragma unroll
+            for (int k = 0; k < V; ++k) if ((moved >> k) & 1u) pf[k] = fill[k];
+    } else {
+        float vel[V], fill[V], comp[V];
+        float* const pf = (float*)fr.fill + s;
+        float* const pv = (float*)fr.vel + s;
+        float* const pc = fr.comp + s;
+        if (whole) { X::load((const float*)pf, fill); X::load((const float*)pc, comp); }
+        else
+#pragma unroll
+            for (int k = 0; k < V; ++k) { fill[k] = (act >> k) & 1u ? pf[k] : 0.0f; comp[k] = (act >> k) & 1u ? pc[k] : 0.0f; }
+        if (a.refresh == 0) {
+            if (whole) X::load((const float*)pv, vel);
+            else
+#pragma unroll
+                for (int k = 0; k < V; ++k) vel[k] = (act >> k) & 1u ? pv[k] : -1.0f;
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+                const uint8_t d = (uint8_t)(dw >> (8 * k));
+                if (!((act >> k) & 1u) || !(d & kPend)) continue;
+                vel[k] = (float)answered_velocity(a, fr, s + k, d, ((const uint32_t*)fr.vel)[s + k]);
+                pv[k] = vel[k];
+            }
+        } else {
+            double mo[V];
+            uint32_t g[V];
+            if (whole) X::load((const uint32_t*)fr.defg + s, g);
+            else
+#pragma unroll
+                for (int k = 0; k < V; ++k) g[k] = (act >> k) & 1u ? fr.defg[s + k] : 0u;
+            if (a.refresh == 2) {
+                if (whole) X::load((const double*)fr.mob + s, mo);
+                else
+#pragma unroll
+                    for (int k = 0; k < V; ++k) mo[k] = (act >> k) & 1u ? fr.mob[s + k] : 0.0;
+            } else {
+                uint32_t r[V];
+                if (whole) X::load((const uint32_t*)fr.rxg + s, r);
+                else
+#pragma unroll
+                    for (int k = 0; k < V; ++k) r[k] = (act >> k) & 1u ? fr.rxg[s + k] : 0u;
+#pragma unroll
+                for (int k = 0; k < V; ++k) {
+                    mo[k] = 0.0;
+                    if (((act >> k) & 1u) && !((dw >> (8 * k)) & kPend))
+                        mo[k] = mobility(a, __longlong_as_double((long long)a.ptab[(unsigned long long)r[k] * a.ndefg + g[k]]));
+                }
+                if (whole) X::store(fr.mob + s, mo);
+                else
+#pragma unroll
+                    for (int k = 0; k < V; ++k) if ((act >> k) & 1u) fr.mob[s + k] = mo[k];
+            }
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+                const uint8_t d = (uint8_t)(dw >> (8 * k));
+                vel[k] = -1.0f;
+                if (!((act >> k) & 1u)) continue;
+                if (d & kPend) vel[k] = (float)answered_velocity(a, fr, s + k, d, ((const uint32_t*)fr.vel)[s + k]);
+                else vel[k] = (float)velocity_from_mobility(a, mo[k], g[k], d & kCodeMask);
+            }
+            if (whole) X::store(pv, vel);
+            else
+#pragma unroll
+                for (int k = 0; k < V; ++k) if ((act >> k) & 1u) pv[k] = vel[k];
+        }
+        uint32_t moved = 0;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            const uint8_t d = (uint8_t)(dw >> (8 * k));
+            if (!((act >> k) & 1u)) continue;
+            if (d & kStale) fr.dir[s + k] = d & kCodeMask;
+            if (vel[k] >= 0.0f) {
+                // Kahan-compensated accumulation of the fill
+                const float inc = vel[k] * a.dtc32;
+                const float y = inc - comp[k];
+                const float t = fill[k] + y;
+                const float c = (t - fill[k]) - y;
+                fill[k] = t; comp[k] = c;
+                moved |= 1u << k;
+                if ((t - c) >= 1.0f) full |= 1u << k;
+            }
+        }
+        if (whole) { if (moved) { X::store(pf, fill); X::store(pc, comp); } }
+        else
+#pragma unroll
+            for (int k = 0; k < V; ++k) if ((moved >> k) & 1u) { pf[k] = fill[k]; pc[k] = comp[k]; }
+    }
+}
+
+template <bool FP32, int ITEMS>
 __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant__ FuseMap map, int base) {
     extern __shared__ __align__(16) char s_raw[];
     FuseShared& sh = *reinterpret_cast<FuseShared*>(s_raw);
@@ -260,17 +521,18 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
     for (uint32_t i = threadIdx.x; i < sizeof(DomainArgs) / 4; i += kFuse)
         ((uint32_t*)&sh.a)[i] = ((const uint32_t*)&c_args[base + dom])[i];
     __syncthreads();
-    const DomainArgs& a = sh.a;
-    if (!a.active) return;
+    const DomainArgs& a = sh.a;                  // with what changes between steps
+    const DomainArgs& cst = c_args[base + dom];   // the rest, by the constant cache: uniform registers, no shared loads
+    if (!cst.active) return;
+    constexpr uint32_t kTile = FuseShape<ITEMS>::kTile, kWords = FuseShape<ITEMS>::kWords;
     DevState* const st = a.st;
     FuseDom* const fd = a.fuse;
     FuseHost* const fh = &a.box->fuse;
     const bool first = rank == 0;
     uint32_t n0 = st->next_never[0], n1 = st->next_never[1];
     uint32_t seq = map.seq[dom] & kCmdSeqMask, arrived = 0;
-    // this lane's direction
-    const int dl = lane < 26 ? lane : 25;
-    const int dx = c_dx[dl], dy = c_dy[dl], dz = c_dz[dl];
+    if (threadIdx.x < 26)
+        sh.dir[threadIdx.x] = (uint32_t)(c_dx[threadIdx.x] + 1) | ((uint32_t)(c_dy[threadIdx.x] + 1) << 2) | ((uint32_t)(c_dz[threadIdx.x] + 1) << 4);
     for (;;) {
         // ---- the host's word for step `seq`
         if (first) {
@@ -336,36 +598,45 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
         __syncthreads();
 
         // ---- A: fill
-        const uint32_t T0 = (n0 + kFuseTile - 1) / kFuseTile, T = T0 + (n1 + kFuseTile - 1) / kFuseTile;
+        const uint32_t T0 = (n0 + kTile - 1) / kTile, T = T0 + (n1 + kTile - 1) / kTile;
         const uint32_t nlt = T > rank ? (T - rank + G - 1) / G : 0u;
-        uint2* const cntA = (uint2*)a.f[0].tcnt;   // per tile (full, INACTIVE)
+        uint2* const cntA = (uint2*)cst.f[0].tcnt;   // per tile (full, INACTIVE)
         uint2* const cntB = cntA + T;              // per tile wins (Inside, Border)
-        const FuseRecs rec{sh, rank, G, T0, n0, nlt};
+        const FuseRecs<ITEMS> rec{sh, rank, G, T0, n0, nlt};
         // the masks of a few tiles stay in shared memory
-        const bool own = nlt * kFuseTileWords <= (uint32_t)kFuse;
+        const bool own = nlt * kWords <= kFuseMask;
+        // the next tile's infector bytes are in flight while this tile's fields are
+        const uint32_t in_tile = (uint32_t)threadIdx.x * ITEMS;
+        uint32_t dirs = 0xFFFFFFFFu;
+        if (nlt) dirs = rank >= T0 ? fuse_dirs<ITEMS>(cst.f[1], (rank - T0) * kTile + in_tile, n1) : fuse_dirs<ITEMS>(cst.f[0], rank * kTile + in_tile, n0);
         for (uint32_t lt = 0; lt < nlt; ++lt) {
-            const uint32_t u = rank + lt * G;
+            const uint32_t u = rank + lt * G, un = u + G;
+            uint32_t next = 0xFFFFFFFFu;
+            if (lt + 1 < nlt) next = un >= T0 ? fuse_dirs<ITEMS>(cst.f[1], (un - T0) * kTile + in_tile, n1) : fuse_dirs<ITEMS>(cst.f[0], un * kTile + in_tile, n0);
             const int L = u >= T0 ? 1 : 0;
             const uint32_t tl = L ? u - T0 : u, n = L ? n1 : n0;
-            const DFront& fr = a.f[L];
-            const uint32_t slot = tl * kFuseTile + (uint32_t)warp * 32u * kFuseItems + (uint32_t)lane;
+            const DFront& fr = cst.f[L];
+            const uint32_t slot = tl * kTile + in_tile;
             uint32_t act, full;
-            fuse_grow<FP32>(a, fr, slot, n, act, full);
-            uint32_t mf = 0, mi = 0;
+            fuse_grow<FP32, ITEMS>(a, fr, slot, dirs, act, full);
+            dirs = next;
+            // 32 / ITEMS lanes share a mask word
+            const uint32_t left = n > slot ? min(n - slot, (uint32_t)ITEMS) : 0u;
+            const uint32_t sh0 = ((uint32_t)lane * ITEMS) & 31u;
+            uint32_t mf = full << sh0, mi = (~act & ((1u << left) - 1u)) << sh0;
 #pragma unroll
-            for (int k = 0; k < kFuseItems; ++k) {
-                const uint32_t f = __ballot_sync(0xFFFFFFFFu, (full >> k) & 1u);
-                const uint32_t i = __ballot_sync(0xFFFFFFFFu, !((act >> k) & 1u) && slot + 32u * (uint32_t)k < n);
-                if (lane == k) { mf = f; mi = i; }
+            for (int o = 1; o < 32 / ITEMS; o <<= 1) {
+                mf |= __shfl_xor_sync(0xFFFFFFFFu, mf, o);
+                mi |= __shfl_xor_sync(0xFFFFFFFFu, mi, o);
             }
-            if (lane < kFuseItems) {
-                const uint32_t wt = (uint32_t)(warp * kFuseItems + lane);
+            if (sh0 == 0u) {
+                const uint32_t wt = in_tile >> 5;
                 if (own) {
-                    sh.fm[lt * kFuseTileWords + wt] = mf;
-                    sh.im[lt * kFuseTileWords + wt] = mi;
+                    sh.fm[lt * kWords + wt] = mf;
+                    sh.im[lt * kWords + wt] = mi;
                 } else {
-                    fr.fmask[tl * kFuseTileWords + wt] = mf;
-                    fr.imask[tl * kFuseTileWords + wt] = mi;
+                    fr.fmask[tl * kWords + wt] = mf;
+                    fr.imask[tl * kWords + wt] = mi;
                 }
             }
         }
@@ -373,26 +644,26 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
         __syncthreads();
         // full cells into records in slot order, tile by tile; the tiles' counts
         uint32_t F = 0;
-        for (uint32_t w0 = 0; w0 < nlt * kFuseTileWords; w0 += kFuse) {
-            const uint32_t wi = w0 + threadIdx.x, lt = wi / kFuseTileWords;
+        for (uint32_t w0 = 0; w0 < nlt * kWords; w0 += kFuse) {
+            const uint32_t wi = w0 + threadIdx.x, lt = wi / kWords;
             uint32_t fw = 0, iw = 0, key0 = 0;
             if (lt < nlt) {
                 const uint32_t u = rank + lt * G;
                 const int L = u >= T0 ? 1 : 0;
-                const uint32_t word = (L ? u - T0 : u) * kFuseTileWords + (wi - lt * kFuseTileWords);
-                fw = own ? sh.fm[wi] : a.f[L].fmask[word];
-                iw = own ? sh.im[wi] : a.f[L].imask[word];
+                const uint32_t word = (L ? u - T0 : u) * kWords + (wi - lt * kWords);
+                fw = own ? sh.fm[wi] : cst.f[L].fmask[word];
+                iw = own ? sh.im[wi] : cst.f[L].imask[word];
                 key0 = (word * 32u) | ((uint32_t)L << 31);
             }
             const uint32_t c = __popc(fw), ci = __popc(iw);
             uint32_t x = c, y = ci, tx, ty;
             block_scan2(sh, x, y, tx, ty);
-            if (lt < nlt && (wi & (kFuseTileWords - 1)) == 0) sh.off[lt] = F + x;
+            if (lt < nlt && (wi & (kWords - 1)) == 0) sh.off[lt] = F + x;
             // the tile's counts: the last of its words knows the sum from the first's prefix
             __syncthreads();
-            if (lt < nlt && (wi & (kFuseTileWords - 1)) == 0) sh.pre[1][lt] = y;
+            if (lt < nlt && (wi & (kWords - 1)) == 0) sh.pre[1][lt] = y;
             __syncthreads();
-            if (lt < nlt && (wi & (kFuseTileWords - 1)) == kFuseTileWords - 1)
+            if (lt < nlt && (wi & (kWords - 1)) == kWords - 1)
                 cntA[rank + lt * G] = make_uint2(F + x + c - sh.off[lt], y + ci - sh.pre[1][lt]);
             uint32_t i = F + x;
             for (uint32_t m = fw; m; m &= m - 1u, ++i) {
@@ -402,32 +673,59 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             F += tx;
         }
         __syncthreads();
-        // the infection attempts: a warp takes 4 full cells at a time, a lane one direction of each
-        for (uint32_t i0 = (uint32_t)warp; i0 < F; i0 += kFuseWarps * 4u) {
-            uint32_t key[4], cell[4], tg[4], gv[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) key[j] = i0 + kFuseWarps * j < F ? rec.key(i0 + kFuseWarps * j) : 0u;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) cell[j] = i0 + kFuseWarps * j < F ? a.f[key[j] >> 31].xyz[key[j] & 0x7FFFFFFFu] : 0u;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                gv[j] = 0xFFFFFFFFu;
-                if (i0 + kFuseWarps * j < F && lane < 26) {
+        // the infection attempts: four lanes a full cell; an interior cell's 8 bricks two a lane, a face cell's directions
+        // 6 or 7 a lane (a warp a cell and a lane a direction spent its time on addresses: 33 us a step of a
+        // 16-domain batch).  The next cells' positions are in flight meanwhile.
+        {
+            auto position = [&](uint32_t i, uint32_t& key) -> uint32_t {
+                if (i >= F) return 0u;
+                key = rec.key(i);
+                return (key >> 31 ? cst.f[1].xyz : cst.f[0].xyz)[key & 0x7FFFFFFFu];
+            };
+            uint32_t i = (uint32_t)warp * 8u + (uint32_t)(lane >> 2), key = 0, key_next = 0;
+            uint32_t cell = position(i, key);
+            for (uint32_t i0 = (uint32_t)warp * 8u; i0 < F; i0 += kFuseWarps * 8u) {
+                const uint32_t in = i + kFuseWarps * 8u, cell_next = position(in, key_next);
+                uint32_t mask = 0;
+                if (i < F) {
+                    const uint32_t ord = ((key & 0x7FFFFFFFu) + (key >> 31 ? n0 : 0u)) * 26u;
                     int x, y, z;
-                    bool inter;
-                    decode(a, cell[j], x, y, z);
-                    if (target_lane(a, (int)(key[j] >> 31), x, y, z, dx, dy, dz, tg[j], inter)) gv[j] = a.grid[tg[j]];
-                }
-            }
+                    decode(cst, cell, x, y, z);
+                    if (x > 0 && y > 0 && z > 0 && x < (int)cst.nx - 1 && y < (int)cst.ny - 1 && z < (int)cst.nz - 1) {
+                        const int b = lane & 3;
+                        const uint32_t w0 = brick_word(cst, x, y, z, b), w1 = brick_word(cst, x, y, z, b + 4);
+                        Brick r0, r1;
+                        load_brick(cst.grid + w0, r0);
+                        load_brick(cst.grid + w1, r1);
+                        mask = claim_brick(cst, x, y, z, b, w0, r0, ord) | claim_brick(cst, x, y, z, b + 4, w1, r1, ord);
+                    } else {
+                        Moore mo;
+                        if (moore_of(cst, (int)(key >> 31), cell, mo)) {
+                            uint32_t tg[7], gv[7];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const bool at = gv[j] < a.ndefg;
-                if (at) {
-                    const uint32_t s = (key[j] & 0x7FFFFFFFu) + (key[j] >> 31 ? n0 : 0u);
-                    atomicMin(&a.claim[tg[j]], s * 26u + (uint32_t)lane);
+                            for (int k = 0; k < 7; ++k) {
+                                const uint32_t d = (uint32_t)(lane & 3) + 4u * (uint32_t)k;
+                                bool inter;
+                                gv[k] = 0xFFFFFFFFu;
+                                if (d < 26u && moore_word(mo, sh.dir[d], tg[k], inter)) gv[k] = cst.grid[tg[k]];
+                            }
+#pragma unroll
+                            for (int k = 0; k < 7; ++k) {
+                                const uint32_t d = (uint32_t)(lane & 3) + 4u * (uint32_t)k;
+                                if (gv[k] >= cst.ndefg) continue;
+                                atomicMin(&cst.claim[tg[k]], ord + d);
+                                mask |= 1u << d;
+                            }
+                        }
+                    }
                 }
-                const uint32_t m = __ballot_sync(0xFFFFFFFFu, at);
-                if (lane == 0 && i0 + kFuseWarps * j < F) { rec.set_win(i0 + kFuseWarps * j, m); rec.set_cell(i0 + kFuseWarps * j, cell[j]); }
+                mask |= __shfl_xor_sync(0xFFFFFFFFu, mask, 1);
+                mask |= __shfl_xor_sync(0xFFFFFFFFu, mask, 2);
+                if (i < F && (lane & 3) == 0) {
+                    rec.set_win(i, mask);
+                    rec.set_cell(i, cell);
+                }
+                i = in; key = key_next; cell = cell_next;
             }
         }
         arrived += G;
@@ -437,9 +735,10 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
         // ---- B: recycle list, wins
         tile_scan(sh, cntA, T, T0, rank, G);
         const uint32_t Ftot = sh.tot[0], F0 = sh.t0[0], I0 = sh.t0[1], I1 = sh.tot[1] - I0;
-        const uint32_t nrec0 = min(I0, a.f[0].reccap), nrec1 = min(I1, a.f[1].reccap);
+        const uint32_t nrec0 = min(I0, cst.f[0].reccap), nrec1 = min(I1, cst.f[1].reccap);
         {
-            // slots that this step cannot hand out are not listed: at most 26 new cells a full cell
+            // slots that this step cannot hand out are not listed: at most 26 new cells a full cell (a count of the
+            // attempts would bound it closer, but took 1 us a step of a small domain)
             const uint32_t most = (uint32_t)min(26ull * Ftot, 0xFFFFFFFFull);
             for (uint32_t lt = 0; lt < nlt; ++lt) {
                 const uint32_t u = rank + lt * G;
@@ -447,17 +746,17 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
                 const uint32_t cap = min(L ? nrec1 : nrec0, most), r0 = sh.pre[1][lt] - (L ? I0 : 0u);
                 if (r0 >= cap) continue;  // uniform over the block
                 // warp w lists the slots of words w and w + kFuseWarps: their ranks from all words' counts
-                const DFront& fr = a.f[L];
-                const uint32_t word0 = (L ? u - T0 : u) * kFuseTileWords;
-                uint32_t iw[kFuseItems], ci[kFuseItems], before = 0;
+                const DFront& fr = cst.f[L];
+                const uint32_t word0 = (L ? u - T0 : u) * kWords;
+                uint32_t iw[ITEMS], ci[ITEMS], before = 0;
 #pragma unroll
-                for (int h = 0; h < kFuseItems; ++h) {
+                for (int h = 0; h < ITEMS; ++h) {
                     const uint32_t k = 32u * (uint32_t)h + (uint32_t)lane;
-                    iw[h] = own ? sh.im[lt * kFuseTileWords + k] : fr.imask[word0 + k];
+                    iw[h] = own ? sh.im[lt * kWords + k] : fr.imask[word0 + k];
                     ci[h] = __popc(iw[h]);
                 }
 #pragma unroll
-                for (int h = 0; h < kFuseItems; ++h) {  // word 32 h + warp
+                for (int h = 0; h < ITEMS; ++h) {  // word 32 h + warp
                     const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, ci[h]);
                     const uint32_t part = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? ci[h] : 0u);
                     const uint32_t wj = __shfl_sync(0xFFFFFFFFu, iw[h], warp);
@@ -467,42 +766,51 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
                 }
             }
         }
-        for (uint32_t i0 = (uint32_t)warp; i0 < F; i0 += kFuseWarps * 4u) {
-            uint32_t key[4], cl[4];
-            bool at[4], tb[4];
+        for (uint32_t i0 = (uint32_t)warp * 8u; i0 < F; i0 += kFuseWarps * 8u) {
+            const uint32_t i = i0 + (uint32_t)(lane >> 2);
+            uint32_t win = 0, tob = 0, key = 0;
+            if (i < F) {
+                key = rec.key(i);
+                const uint32_t mask = rec.win(i);
+                Moore mo;
+                if (mask && moore_of(cst, (int)(key >> 31), rec.cell(i), mo)) {
+                    const uint32_t s = (key & 0x7FFFFFFFu) + (key >> 31 ? n0 : 0u);
+                    // the lane's share of the attempts made, their claims in flight together
+                    uint32_t m = mask & (0x01111111u << (lane & 3)), cl[7], at[7], inm = 0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                at[j] = false; tb[j] = false; cl[j] = kClaimFree; key[j] = 0u;
-                if (i0 + kFuseWarps * j < F) {
-                    key[j] = rec.key(i0 + kFuseWarps * j);
-                    at[j] = (rec.win(i0 + kFuseWarps * j) >> lane) & 1u;
-                    if (at[j]) {
-                        const int L = (int)(key[j] >> 31);
-                        int x, y, z;
-                        decode(a, rec.cell(i0 + kFuseWarps * j), x, y, z);
-                        uint32_t t;
-                        bool inter;
-                        target_lane(a, L, x, y, z, dx, dy, dz, t, inter);
-                        cl[j] = a.claim[t];
-                        // Inside full cells near a face infect into the Border list (SCORE_Kernel.cpp:4606-4609);
-                        // Border full cells send strictly interior targets to the Inside list (:4387)
-                        const bool allB = !(x > 1 && x < (int)a.nx - 2 && y > 1 && y < (int)a.ny - 2 && z > 1 && z < (int)a.nz - 2);
-                        tb[j] = L == 0 ? allB : !inter;
+                    for (int k = 0; k < 7; ++k) {
+                        at[k] = 0xFFFFFFFFu; cl[k] = kClaimFree;
+                        if (m) {
+                            at[k] = (uint32_t)(__ffs(m) - 1);
+                            m &= m - 1u;
+                            uint32_t t;
+                            bool inter;
+                            moore_word(mo, sh.dir[at[k]], t, inter);
+                            cl[k] = cst.claim[t];
+                            inm |= (inter ? 1u : 0u) << k;
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 7; ++k) {
+                        if (at[k] < 26u && cl[k] == s * 26u + at[k]) {
+                            win |= 1u << at[k];
+                            // Inside full cells near a face infect into the Border list (SCORE_Kernel.cpp:4606-4609);
+                            // Border full cells send strictly interior targets to the Inside list (:4387)
+                            if (key >> 31 ? !((inm >> k) & 1u) : mo.near) tob |= 1u << at[k];
+                        }
                     }
                 }
             }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t s = (key[j] & 0x7FFFFFFFu) + (key[j] >> 31 ? n0 : 0u);
-                const bool won = at[j] && cl[j] == s * 26u + (uint32_t)lane;
-                const uint32_t win = __ballot_sync(0xFFFFFFFFu, won), tob = __ballot_sync(0xFFFFFFFFu, won && tb[j]);
-                if (lane == 0 && i0 + kFuseWarps * j < F) {
-                    rec.set_win(i0 + kFuseWarps * j, win);
-                    rec.set_tob(i0 + kFuseWarps * j, tob);
-                    const uint32_t lt = rec.tile(i0 + kFuseWarps * j, key[j]), cB = __popc(tob), cA = __popc(win) - cB;
-                    if (cA) atomicAdd(&sh.tw[0][lt], cA);
-                    if (cB) atomicAdd(&sh.tw[1][lt], cB);
-                }
+            win |= __shfl_xor_sync(0xFFFFFFFFu, win, 1);
+            tob |= __shfl_xor_sync(0xFFFFFFFFu, tob, 1);
+            win |= __shfl_xor_sync(0xFFFFFFFFu, win, 2);
+            tob |= __shfl_xor_sync(0xFFFFFFFFu, tob, 2);
+            if (i < F && (lane & 3) == 0) {
+                rec.set_win(i, win);
+                rec.set_tob(i, tob);
+                const uint32_t lt = rec.tile(i, key), cB = __popc(tob), cA = __popc(win) - cB;
+                if (cA) atomicAdd(&sh.tw[0][lt], cA);
+                if (cB) atomicAdd(&sh.tw[1][lt], cB);
             }
         }
         __syncthreads();
@@ -543,10 +851,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
                 const uint32_t slot = key & 0x7FFFFFFFu;
                 rs = fr.rxg[slot];
                 gs = fr.defg[slot];
-                if (win) {
-                    if (!FP32) over = __dsub_rn(((const double*)fr.fill)[slot], 1.0);
-                    else over = (double)((((const float*)fr.fill)[slot] - 1.0f) - fr.comp[slot]);
-                }
+                if (win) over = full_over<FP32>(fr, slot);
             }
             // the grains' counts: the atomic's answer is looked at after the new cells
             const uint32_t has = __ballot_sync(0xFFFFFFFFu, i < F);
@@ -554,10 +859,10 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             if (has) {
                 const uint32_t mr = __match_any_sync(0xFFFFFFFFu, i < F ? rs : 0xFFFFFFFFu) & has;
                 const uint32_t mg = __match_any_sync(0xFFFFFFFFu, i < F ? gs : 0xFFFFFFFFu) & has;
-                if (i < F && (__ffs(mr) - 1) == lane) atomicAdd(&a.rxg_cnt[rs], (uint32_t)__popc(mr));
+                if (i < F && (__ffs(mr) - 1) == lane) atomicAdd(&cst.rxg_cnt[rs], (uint32_t)__popc(mr));
                 if (i < F && (__ffs(mg) - 1) == lane) {
                     gk = (uint32_t)__popc(mg);
-                    gold = atomicSub(&a.defg_cnt[gs], gk);
+                    gold = atomicSub(&cst.defg_cnt[gs], gk);
                 }
             }
             const uint32_t cB = __popc(tob), cA = __popc(win) - cB;
@@ -572,42 +877,47 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
                 sh.c_cell[threadIdx.x] = cell | (key & 0x80000000u);
                 sh.c_rs[threadIdx.x] = rs;
                 sh.c_over[threadIdx.x] = over;
-                uint32_t q = xa + xb;
-                for (uint32_t m = win; m; m &= m - 1u) sh.wl[q++] = (uint16_t)((threadIdx.x << 5) | (uint32_t)(__ffs(m) - 1));
             }
-            __syncthreads();
+            // the chunk's new cells in record and direction order, kFuseWins at a time
             const uint32_t W = ta + tb;
-            for (uint32_t k = threadIdx.x; k < W; k += kFuse) {
-                const uint32_t e = sh.wl[k], t = e >> 5;
-                const int d = (int)(e & 31u);
-                const uint32_t m = sh.c_win[t], tbm = sh.c_tob[t], below = m & ((1u << d) - 1u);
-                const int D = (tbm >> d) & 1u;
-                const uint32_t r = D ? sh.c_rB[t] + __popc(below & tbm) : sh.c_rA[t] + __popc(below & ~tbm);
-                const uint32_t sc = sh.c_cell[t];
-                int x, y, z;
-                decode(a, sc & 0x7FFFFFFFu, x, y, z);
-                uint32_t tgt;
-                bool inter;
-                target_of(a, (int)(sc >> 31), x, y, z, d, tgt, inter);
-                const uint32_t gt = a.grid[tgt];
-                const DFront& dst = a.f[D];
-                const uint32_t nrec = D ? nrec1 : nrec0;
-                const uint32_t ns = r < nrec ? dst.recyc[r] : (D ? n1 : n0) + (r - nrec);
-                if (ns >= dst.cap) { atomicOr(&st->err, kErrCapacity); continue; }
-                if (D == 1 && a.border_policy == 0 && r >= nrec && ns >= a.border_ref_cap) atomicOr(&st->err, kErrBorderRef);
-                new_cell<FP32>(a, dst, ns, tgt, gt, sh.c_rs[t], sh.c_over[t], d, pmax, ntag);
+            for (uint32_t w0 = 0; w0 < W; w0 += kFuseWins) {
+                if (w0) __syncthreads();
+                uint32_t q = xa + xb;
+                for (uint32_t m = win; m; m &= m - 1u, ++q)
+                    if (q - w0 < kFuseWins) sh.wl[q - w0] = (uint16_t)((threadIdx.x << 5) | (uint32_t)(__ffs(m) - 1));
+                __syncthreads();
+                for (uint32_t k = threadIdx.x; k < min(W - w0, kFuseWins); k += kFuse) {
+                    const uint32_t e = sh.wl[k], t = e >> 5;
+                    const int d = (int)(e & 31u);
+                    const uint32_t m = sh.c_win[t], tbm = sh.c_tob[t], below = m & ((1u << d) - 1u);
+                    const int D = (tbm >> d) & 1u;
+                    const uint32_t r = D ? sh.c_rB[t] + __popc(below & tbm) : sh.c_rA[t] + __popc(below & ~tbm);
+                    const uint32_t sc = sh.c_cell[t];
+                    int x, y, z;
+                    decode(cst, sc & 0x7FFFFFFFu, x, y, z);
+                    uint32_t tgt;
+                    bool inter;
+                    target_of(cst, (int)(sc >> 31), x, y, z, d, tgt, inter);
+                    const uint32_t gt = cst.grid[tgt];
+                    const DFront& dst = a.f[D];
+                    const uint32_t nrec = D ? nrec1 : nrec0;
+                    const uint32_t ns = r < nrec ? dst.recyc[r] : (D ? n1 : n0) + (r - nrec);
+                    if (ns >= dst.cap) { atomicOr(&st->err, kErrCapacity); continue; }
+                    if (D == 1 && cst.border_policy == 0 && r >= nrec && ns >= cst.border_ref_cap) atomicOr(&st->err, kErrBorderRef);
+                    new_cell<FP32>(a, dst, ns, tgt, gt, sh.c_rs[t], sh.c_over[t], d, pmax, ntag);
+                }
             }
             if (i < F) {  // the full cell is now recrystallized
                 const DFront& src = a.f[key >> 31];
                 const uint32_t slot = key & 0x7FFFFFFFu;
-                a.grid[cell] = a.ndefg + rs;
+                cst.grid[cell] = cst.ndefg + rs;
                 src.dir[slot] = kInactive;
                 if (!FP32) ((double*)src.fill)[slot] = 0.0;
                 else { ((float*)src.fill)[slot] = 0.0f; src.comp[slot] = 0.0f; }
             }
             if (gk && gold == gk) {
                 const uint32_t q = atomicAdd(&st->ndepleted, 1u);
-                if (q < a.ndefg) a.depleted[q] = gs;
+                if (q < cst.ndefg) cst.depleted[q] = gs;
             }
             ca += ta; cb += tb;
             __syncthreads();
@@ -620,15 +930,15 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
         if (W0 > nrec0) n0 += W0 - nrec0;
         if (W1 > nrec1) n1 += W1 - nrec1;
         bool over_cap = false;
-        if (n0 > a.f[0].cap) { n0 = a.f[0].cap; over_cap = true; }
-        if (n1 > a.f[1].cap) { n1 = a.f[1].cap; over_cap = true; }
+        if (n0 > cst.f[0].cap) { n0 = cst.f[0].cap; over_cap = true; }
+        if (n1 > cst.f[1].cap) { n1 = cst.f[1].cap; over_cap = true; }
 
         // ---- D: the step to the host
         if (first) {
-            HostBox* const box = a.box;
-            const uint32_t nm = min(min(__ldcg(&st->nmiss), a.misscap), kBoxMiss), nd = min(min(__ldcg(&st->ndepleted), a.ndefg), kBoxDep);
-            for (uint32_t i = threadIdx.x; i < nm; i += kFuse) box->miss[i] = __ldcg(&a.miss[i]);
-            for (uint32_t i = threadIdx.x; i < nd; i += kFuse) box->depleted[i] = __ldcg(&a.depleted[i]);
+            HostBox* const box = cst.box;
+            const uint32_t nm = min(min(__ldcg(&st->nmiss), cst.misscap), kBoxMiss), nd = min(min(__ldcg(&st->ndepleted), cst.ndefg), kBoxDep);
+            for (uint32_t i = threadIdx.x; i < nm; i += kFuse) box->miss[i] = __ldcg(&cst.miss[i]);
+            for (uint32_t i = threadIdx.x; i < nd; i += kFuse) box->depleted[i] = __ldcg(&cst.depleted[i]);
             if (threadIdx.x == 0) {
                 DevState v;
                 v.next_never[0] = n0; v.next_never[1] = n1;

@@ -735,8 +735,9 @@ struct Engine {
         args_dirty = true;
         int coop = 0;
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_steps_fused<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FuseShared));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_steps_fused<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FuseShared));
+        for (const void* k : {(const void*)k_steps_fused<false, 2>, (const void*)k_steps_fused<true, 2>, (const void*)k_steps_fused<false, 4>,
+                              (const void*)k_steps_fused<true, 4>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FuseShared));
         fuse = e == cudaSuccess && coop != 0;
         fuse_sms = sms;
         return e == cudaSuccess ? SCORE_OK : SCORE_ERR_CUDA;
@@ -1728,14 +1729,18 @@ int Engine::mark_run_end() {
 namespace {
 
 // Slots of a domain's front up to which its steps run inside one launch.  A fused step saves the separate
-// kernels' fixed cost (about 50 us) but streams a large front at half their occupancy.  Measured per run,
-// limits of 0 / 1 / 2 / 4 / 8 M slots: FP64 384^3 rolled sheet 68.2 / 68.5 / 68.2 / 69.2 / 83.5 ms, FP64 512^3
-// 116.9 / 115.8 / 114.5 / 114.8 / 115.3, FP32 384^3 with recovery 210.6 / 180.1 / 172.5 / 151.4 / 149.6, batch of
-// 12 FP64 84.5 / 71.0 / 64.0 / 64.9 / 64.5.
-constexpr uint64_t kFuseSlots = (uint64_t)kFuseMaxTiles * kFuseTile / 2;
+// kernels' fixed cost (about 50 us) but streams a large front with half their loads in flight.  Measured per run,
+// limits of 2 / 4 / 8 / 14 M slots: FP64 384^3 rolled sheet 67.9 / 68.1 / 63.5 / 63.6 ms, the same with few cells in
+// motion for 2,000 steps 235 / 236 / 171 / 171, FP64 512^3 104.3 / 103.7 / 103.6 / 105.9, FP32 384^3 with recovery
+// 160 / 132 / 131 / 131 (211 with none).
+constexpr uint64_t kFuseSlots = 8ull << 20;
+// Slots a block from which a thread takes 4 slots a tile instead of 2: fewer, wider accesses (16-domain batch: fill
+// 42 us a step with 2, 23 with 4), but half the tiles to spread over the blocks.
+constexpr uint64_t kFuseWide = 4096;
 
-uint32_t fuse_tiles(const score_ctx* c) {
-    return (c->next_never[0] + kFuseTile - 1) / kFuseTile + (c->next_never[1] + kFuseTile - 1) / kFuseTile;
+uint32_t fuse_tiles(const score_ctx* c, int items) {
+    const uint32_t tile = (uint32_t)(kFuse * items);
+    return (c->next_never[0] + tile - 1) / tile + (c->next_never[1] + tile - 1) / tile;
 }
 
 FusePay fuse_pay(const score_ctx* c) {
@@ -1786,7 +1791,7 @@ bool Engine::fused_ok() const {
     for (const score_ctx* c : dom) {
         if (!c->running) continue;
         ++nrun;
-        tiles += fuse_tiles(c);
+        tiles += fuse_tiles(c, 4);
         if ((uint64_t)c->next_never[0] + c->next_never[1] > kFuseSlots) return false;
     }
     // a domain's blocks follow its share of the tiles: kFuseMaxLocal tiles a block with room to grow
@@ -1800,6 +1805,11 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
     cudaSetDevice(device);
     const auto t0 = std::chrono::steady_clock::now();
     const int n = (int)dom.size();
+    uint64_t slots = 0;
+    for (const score_ctx* c : dom)
+        if (c->running) slots += (uint64_t)c->next_never[0] + c->next_never[1];
+    // 4 slots a thread and tile once every block has several tiles of 2
+    const int items = slots >= kFuseWide * (uint64_t)fuse_sms ? 4 : 2;
     std::vector<FuseServe> sv;
     FuseMap map{};
     uint64_t work = 0;
@@ -1813,7 +1823,7 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
         FuseServe f;
         f.c = c; f.i = (size_t)i;
         sv.push_back(f);
-        work += 2ull * fuse_tiles(c) + 8;
+        work += 2ull * fuse_tiles(c, items) + 8;
     }
     const auto t_pre = std::chrono::steady_clock::now();
     tm.pre_ms += std::chrono::duration<double, std::milli>(t_pre - t0).count();
@@ -1825,7 +1835,7 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
         for (int i = 0; i < n; ++i) {
             map.first[i] = (uint16_t)total;
             if (k < sv.size() && sv[k].i == (size_t)i) {
-                const uint32_t want = 2 * fuse_tiles(sv[k].c) + 8;
+                const uint32_t want = 2 * fuse_tiles(sv[k].c, items) + 8;
                 sv[k].blocks = std::min(want, 1u + (uint32_t)((uint64_t)spare * want / work));
                 total += sv[k].blocks;
                 map.seq[i] = sv[k].c->fuse_seq;
@@ -1858,7 +1868,8 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
     }
     if (e == cudaSuccess) {
         void* args[] = {(void*)&map, (void*)&base};
-        const void* k = fp32 ? (const void*)k_steps_fused<true> : (const void*)k_steps_fused<false>;
+        const void* k = items == 4 ? (fp32 ? (const void*)k_steps_fused<true, 4> : (const void*)k_steps_fused<false, 4>)
+                                   : (fp32 ? (const void*)k_steps_fused<true, 2> : (const void*)k_steps_fused<false, 2>);
         e = cudaLaunchCooperativeKernel(k, dim3(total), dim3(kFuse), args, sizeof(FuseShared), stream);
     }
     if (e != cudaSuccess) {
@@ -1938,7 +1949,7 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
         f.status = finish_step(f);
         const double xt = x_target < 0 ? c->prm.xmax : x_target;
         const bool needs = f.status == SCORE_OK && (c->log_info.size() != logged || fuse_needs_stream(c) ||
-                           (uint64_t)c->next_never[0] + c->next_never[1] > kFuseSlots || fuse_tiles(c) > kFuseMaxLocal * f.blocks);
+                           (uint64_t)c->next_never[0] + c->next_never[1] > kFuseSlots || fuse_tiles(c, items) > std::min(kFuseMaxLocal * f.blocks, kFuseMaxTiles - 512));
         if (f.status != SCORE_OK || needs) stop.store(true, std::memory_order_relaxed);
         if (f.status != SCORE_OK || needs || one || domain_done(c, xt) || (max_steps && done[f.i] >= max_steps) ||
             stop.load(std::memory_order_relaxed)) {

@@ -197,7 +197,9 @@ __device__ __forceinline__ double mobility(const DomainArgs& a, double P) {
 }
 // velocity factor (m p) f_geo, or -1 when the driving force is not above 5e-16
 __device__ __forceinline__ double velocity_from_force(double m, double p, int code) {
-    if (!(p > 5.0e-16)) return -1.0;
+    // p > 5e-16 by integers (an FP64 compare takes the FP64 pipe, 1/64 rate); a NaN is not above it
+    const long long b = __double_as_longlong(p);
+    if (!(b > __double_as_longlong(5.0e-16) && b <= 0x7FF0000000000000ll)) return -1.0;
     return __dmul_rn(__dmul_rn(m, p), c_sf[code]);
 }
 __device__ __forceinline__ double velocity_from_mobility(const DomainArgs& a, double m, uint32_t defg, int code) {
@@ -1309,6 +1311,45 @@ __device__ __forceinline__ uint32_t claim_plane(const DomainArgs& a, int x, int 
     return mask;
 }
 
+// One of the 8 bricks around an interior cell (x, y, z), the 32 bytes by one load: the lower (0) or upper (1) brick of
+// the two that x - 1 .. x + 1 touch, and so on for y (bit 1) and z (bit 2).
+struct Brick { uint32_t v[8]; };
+__device__ __forceinline__ uint32_t brick_word(const DomainArgs& a, int x, int y, int z, int b) {
+    return ((((uint32_t)((z - 1) >> 1) + (uint32_t)(b >> 2)) * a.gby + (uint32_t)((y - 1) >> 1) + (uint32_t)((b >> 1) & 1)) * a.gbx +
+            (uint32_t)((x - 1) >> 1) + (uint32_t)(b & 1)) << 3;
+}
+__device__ __forceinline__ void load_brick(const uint32_t* p, Brick& r) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
+                 : "l"(p));
+}
+// The attempts of the cell on the brick's words that are its neighbours and still deformed, with ordinals key + d;
+// returns their directions' bits.  The reference's order of directions, by rows of constant dy and dz: d = row + dx + 1,
+// without the cell itself in its own row.
+__device__ __forceinline__ uint32_t claim_brick(const DomainArgs& a, int x, int y, int z, int b, uint32_t word, const Brick& r, uint32_t key) {
+    constexpr unsigned long long kRows = 11ull | 14ull << 5 | 8ull << 10 | 0ull << 15 | 3ull << 20 | 5ull << 25 | 17ull << 30 | 20ull << 35 | 23ull << 40;
+    // offset of the brick's first cell along each axis: -2 or -1 for the lower brick, 0 or 1 for the upper
+    const int dx0 = 2 * (b & 1) - 2 + (x & 1), dy0 = (b & 2) - 2 + (y & 1), dz0 = 2 * (b >> 2) - 2 + (z & 1);
+    uint32_t mask = 0;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {  // rows of two words
+        const int dy = dy0 + (w & 1), dz = dz0 + (w >> 1);
+        const bool row = (uint32_t)(dy + 1) <= 2u && (uint32_t)(dz + 1) <= 2u;
+        const bool own = dy == 0 && dz == 0;
+        const uint32_t rb = (uint32_t)(kRows >> (5 * (3 * (dz + 1) + dy + 1) & 63)) & 31u;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int dx = dx0 + k;
+            const uint32_t d = rb + (own ? (dx > 0 ? 1u : 0u) : (uint32_t)(dx + 1));
+            if (row && (uint32_t)(dx + 1) <= 2u && !(own && dx == 0) && r.v[2 * w + k] < a.ndefg) {
+                atomicMin(&a.claim[word + (uint32_t)(2 * w + k)], key + d);
+                mask |= 1u << d;
+            }
+        }
+    }
+    return mask;
+}
+
 // full cells of a domain this step (Inside list first); 0 when the 32-bit attempt
 // ordinal 26 f + d could overflow (flagged)
 __device__ __forceinline__ uint32_t full_cells(const DomainArgs& a) {
@@ -1343,26 +1384,21 @@ __global__ void __launch_bounds__(kBlock, 2) k_claim(int base, int ndom) {
         uint32_t mask;
         if (f < F0) {
             // an Inside cell (strictly interior, every list insertion checks it): its neighbourhood
-            // spans 8 bricks; all 26 grid reads in flight before the first claim
+            // spans 8 bricks, one 32-byte load each, all in flight before the first claim (26 word loads a
+            // cell took 26 passes of the L1's tag stage a cell instead of 8)
             const uint32_t cell = a.f[0].xyz[a.f[0].full[f]];
             a.fcell[f] = cell;
             int x, y, z;
             decode(a, cell, x, y, z);
-            uint32_t gv[26];
-#pragma unroll
-            for (int d = 0; d < 26; ++d) {
-                const uint32_t t = gindex(a, (uint32_t)(x + c_dx[d]), (uint32_t)(y + c_dy[d]), (uint32_t)(z + c_dz[d]));
-                gv[d] = t < a.ncells ? a.grid[t] : 0xFFFFFFFFu;
-            }
             mask = 0;
+            if (x < 1 || y < 1 || z < 1 || x > (int)a.nx - 2 || y > (int)a.ny - 2 || z > (int)a.nz - 2) {
+                atomicOr(&a.st->err, kErrBounds);
+            } else {
+                Brick r[8];
 #pragma unroll
-            for (int d = 0; d < 26; ++d) {
-                const uint32_t t = gindex(a, (uint32_t)(x + c_dx[d]), (uint32_t)(y + c_dy[d]), (uint32_t)(z + c_dz[d]));
-                if (t >= a.ncells) atomicOr(&a.st->err, kErrBounds);
-                else if (gv[d] < a.ndefg) {
-                    atomicMin(&a.claim[t], f * 26u + (uint32_t)d);
-                    mask |= 1u << d;
-                }
+                for (int b = 0; b < 8; ++b) load_brick(a.grid + brick_word(a, x, y, z, b), r[b]);
+#pragma unroll
+                for (int b = 0; b < 8; ++b) mask |= claim_brick(a, x, y, z, b, brick_word(a, x, y, z, b), r[b], f * 26u);
             }
         } else {
             const uint32_t cell = a.f[1].xyz[a.f[1].full[f - F0]];
