@@ -330,64 +330,72 @@ __global__ void __launch_bounds__(kBlock) k_area_sum(uint32_t* hist, uint32_t nr
 }
 
 // ---- ensemble post-processing (SCORE_SolitaryUnitAveraging.cpp) of the grain-evolution logs ----
+// caHdl::get_interpCellCount (SCORE_SolitaryUnitAveraging.cpp:1304-1365) of a grain at time `when`: its final count at
+// or after the end of the run, its first count at or before the first snapshot, its last after the last one, else
+//   c1 + ((when - t1) * ((c2 - c1) / (t2 - t1)))
+// between the snapshots around it.  The slope belongs to the grain and the interval, not to the time: k_rediscr_rows
+// makes (c1, slope) once a grain and interval, and a time slot costs a product and a sum on the FP64 pipe (1/64
+// rate), where the division made it ten.  A row with slope 0 is the count itself.
 struct EvoDev {
     const double* t;              // snapshot times
     const uint32_t* counts;       // nsnap x (ndefg + nrxg)
     const uint32_t* fin_defg;     // counts at the end of the run
     const uint32_t* fin_rxg;
-    const uint32_t* cls;          // orientation class of every grain (macrotexture), or null
-    uint32_t ndefg, nrxg, nsnap, pad;
+    const uint32_t* order;        // grains by class, in grain order within a class (macrotexture), or null: 0, 1, ...
+    const uint32_t* first;        // first place of each class in that order, nclass + 1
+    double2* rows;                // (nsnap + 2) x ngr: before the first snapshot, each interval, after the last, the end
+    uint32_t ndefg, nrxg, nsnap, ngr;
     double tsimend, nboxvol;
 };
-// caHdl::get_interpCellCount (SCORE_SolitaryUnitAveraging.cpp:1304-1365) for grain `id`, with the
-// snapshot index i of `when` (first snapshot at or after it) found once per time
-__device__ __forceinline__ double interp_count(const EvoDev& e, uint32_t id, double when, uint32_t i) {
+__global__ void __launch_bounds__(256) k_rediscr_rows(const EvoDev* doms) {
+    const EvoDev e = doms[blockIdx.y];
     const uint32_t G = e.ndefg + e.nrxg;
-    if (when >= e.tsimend) return (double)(id < e.ndefg ? e.fin_defg[id] : e.fin_rxg[id - e.ndefg]);
-    if (i > 0 && i < e.nsnap) {
-        const double ti1 = e.t[i - 1], cnti1 = (double)e.counts[(uint64_t)(i - 1) * G + id];
-        const double ti = e.t[i], cnti = (double)e.counts[(uint64_t)i * G + id];
-        return __dadd_rn(cnti1, __dmul_rn(__dsub_rn(when, ti1), __ddiv_rn(__dsub_rn(cnti, cnti1), __dsub_rn(ti, ti1))));
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < e.ngr; q += gridDim.x * blockDim.x) {
+        const uint32_t id = e.order ? e.order[q] : q;
+        double c1 = (double)e.counts[id], t1 = e.t[0];
+        e.rows[q] = make_double2(c1, 0.0);
+        for (uint32_t i = 1; i < e.nsnap; ++i) {
+            const double c2 = (double)e.counts[(uint64_t)i * G + id], t2 = e.t[i];
+            // equal counts: the quotient is 0 (times ascend), no division
+            e.rows[(uint64_t)i * e.ngr + q] = make_double2(c1, c2 == c1 ? 0.0 : __ddiv_rn(__dsub_rn(c2, c1), __dsub_rn(t2, t1)));
+            c1 = c2; t1 = t2;
+        }
+        e.rows[(uint64_t)e.nsnap * e.ngr + q] = make_double2(c1, 0.0);
+        e.rows[(uint64_t)(e.nsnap + 1) * e.ngr + q] = make_double2((double)(id < e.ndefg ? e.fin_defg[id] : e.fin_rxg[id - e.ndefg]), 0.0);
     }
-    if (i == 0) return (double)e.counts[id];
-    return (double)e.counts[(uint64_t)(e.nsnap - 1) * G + id];
 }
-__device__ __forceinline__ uint32_t snap_index(const EvoDev& e, double when) {
-    uint32_t i = 0;
-    while (i < e.nsnap && e.t[i] < when) ++i;
-    return i;
-}
-// one thread per (domain, time slot): the domain's interpolated deformed volume, summed over its
-// grains in order (postprocess_rediscr_kinetics, :546-600), as box volume minus it
-__global__ void k_rediscr_kinetics(const EvoDev* doms, uint32_t ndom, const double* when, uint32_t nslots, double* per_dom) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= ndom * nslots) return;
-    const uint32_t d = k / nslots, n = k - d * nslots;
-    const EvoDev e = doms[d];
-    const double w = when[n];
-    const uint32_t i = snap_index(e, w);
-    double dv = 0.0;
-    for (uint32_t g = 0; g < e.ndefg; ++g) dv = __dadd_rn(dv, interp_count(e, g, w, i));
-    per_dom[k] = __dsub_rn(e.nboxvol, dv);
-}
-// one thread per (domain, time slot): interpolated volume per orientation class, deformed grains then
-// rx grains in order (postprocess_rediscr_macrotexture, :673-747); [domain][slot][class]
+// One thread per (domain, class, time slot), a warp's slots neighbours in time, so that they mostly read the same row:
+// the class's grains summed in order (postprocess_rediscr_kinetics, :546-600: one class, the deformed grains, as
+// box volume minus the sum; postprocess_rediscr_macrotexture, :673-747).  What bounds it is the FP64 pipe and the
+// chain of sums: 16 grains' rows are in flight at a time, and a grain that is not there in the interval costs no
+// FP64 operation (x + 0 is x for the sums here, which are never -0).
 constexpr uint32_t kMaxClasses = 32;
-__global__ void k_rediscr_texture(const EvoDev* doms, uint32_t ndom, const double* when, uint32_t nslots, uint32_t nclass,
-                                  double* per_dom) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= ndom * nslots) return;
-    const uint32_t d = k / nslots, n = k - d * nslots;
-    const EvoDev e = doms[d];
+__global__ void __launch_bounds__(32) k_rediscr_sum(const EvoDev* doms, const double* when, uint32_t nslots, uint32_t nclass, int kinetics,
+                                                    double* per_dom) {
+    const EvoDev e = doms[blockIdx.z];
+    const uint32_t c = blockIdx.y, n = blockIdx.x * 32u + threadIdx.x;
+    if (n >= nslots) return;
     const double w = when[n];
-    const uint32_t i = snap_index(e, w);
-    double acc[kMaxClasses];
-    for (uint32_t c = 0; c < nclass; ++c) acc[c] = 0.0;
-    for (uint32_t g = 0; g < e.ndefg + e.nrxg; ++g) {
-        const uint32_t c = e.cls[g];
-        acc[c] = __dadd_rn(acc[c], interp_count(e, g, w, i));
+    uint32_t r = 0;
+    while (r < e.nsnap && e.t[r] < w) ++r;  // the first snapshot at or after it
+    double dt = 0.0;
+    if (r > 0 && r < e.nsnap) dt = __dsub_rn(w, e.t[r - 1]);
+    if (w >= e.tsimend) { r = e.nsnap + 1; dt = 0.0; }
+    const uint32_t lo = kinetics ? 0u : e.first[c], hi = kinetics ? e.ndefg : e.first[c + 1];
+    const double2* row = e.rows + (uint64_t)r * e.ngr;
+    constexpr uint32_t U = 16;
+    double acc = 0.0;
+    for (uint32_t g = lo; g < hi; g += U) {
+        double2 v[U];
+#pragma unroll
+        for (uint32_t k = 0; k < U; ++k) v[k] = g + k < hi ? __ldg(&row[g + k]) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (uint32_t k = 0; k < U; ++k) {
+            if (__double_as_longlong(v[k].y) != 0) acc = __dadd_rn(acc, __dadd_rn(v[k].x, __dmul_rn(dt, v[k].y)));
+            else if (__double_as_longlong(v[k].x) != 0) acc = __dadd_rn(acc, v[k].x);
+        }
     }
-    for (uint32_t c = 0; c < nclass; ++c) per_dom[(uint64_t)k * nclass + c] = acc[c];
+    per_dom[((uint64_t)blockIdx.z * nslots + n) * nclass + c] = kinetics ? __dsub_rn(e.nboxvol, acc) : acc;
 }
 // ensemble sums over the domains in order, one thread per output value
 __global__ void k_rediscr_ensemble(const double* per_dom, uint32_t ndom, uint32_t m, double* out) {
@@ -2261,55 +2269,71 @@ int rediscr(const std::vector<score_ctx*>& doms, uint32_t nslots, const uint32_t
         const cudaError_t e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) { err = cudaGetErrorString(e); return SCORE_ERR_CUDA; }
     }
-    const uint32_t ndom = (uint32_t)doms.size(), m = cls ? nslots * nclass : nslots;
-    // one device block: domain descriptors, snapshot times, slot times, classes, per-domain and ensemble sums
-    const size_t b_evo = ndom * sizeof(EvoDev), b_t = ntimes * 8, b_w = (size_t)nslots * 8, b_c = cls ? ncls * 4 : 0;
+    const uint32_t ndom = (uint32_t)doms.size(), m = cls ? nslots * nclass : nslots, nc = cls ? nclass : 1u;
+    // one block of the first domain's staging buffer: what the host sends (descriptors, snapshot times, slot times,
+    // grains by class), then rows and sums
+    size_t nrows = 0, maxgr = 0;
+    for (score_ctx* c : doms) {
+        const size_t ngr = cls ? (size_t)c->ndefg + c->nrxg : c->ndefg;
+        nrows += (c->log_info.size() + 2) * ngr;
+        maxgr = std::max(maxgr, ngr);
+    }
+    const size_t b_evo = ndom * sizeof(EvoDev), b_t = ntimes * 8, b_w = (size_t)nslots * 8, b_o = cls ? ncls * 4 : 0, b_f = cls ? (size_t)ndom * (nc + 1) * 4 : 0;
     const size_t b_pd = (size_t)ndom * m * 8, b_out = (size_t)m * 8;
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    const size_t total = up(b_evo) + up(b_t) + up(b_w) + up(b_c) + up(b_pd) + up(b_out);
-    char* blk = nullptr;
-    cudaError_t e = cudaMalloc((void**)&blk, total);
-    if (e != cudaSuccess) { err = "post-processing buffers"; return SCORE_ERR_NOMEM; }
-    EvoDev* d_evo = (EvoDev*)blk;
-    double* d_t = (double*)(blk + up(b_evo));
-    double* d_w = (double*)((char*)d_t + up(b_t));
-    uint32_t* d_c = (uint32_t*)((char*)d_w + up(b_w));
-    double* d_pd = (double*)((char*)d_c + up(b_c));
-    double* d_out = (double*)((char*)d_pd + up(b_pd));
-    std::vector<EvoDev> evo(ndom);
-    std::vector<double> times;
-    times.reserve(ntimes);
-    size_t toff = 0, coff = 0;
+    const size_t o_t = up(b_evo), o_w = o_t + up(b_t), o_o = o_w + up(b_w), o_f = o_o + up(b_o), sent = o_f + up(b_f);
+    const size_t o_pd = sent + up(nrows * 16), o_out = o_pd + up(b_pd);
+    if (!doms[0]->stage(o_out + up(b_out))) { err = "post-processing buffers"; return SCORE_ERR_NOMEM; }
+    char* const blk = (char*)doms[0]->d_stage;
+    std::vector<char> host(sent);
+    EvoDev* evo = (EvoDev*)host.data();
+    double* times = (double*)(host.data() + o_t);
+    uint32_t* order = (uint32_t*)(host.data() + o_o);
+    uint32_t* first = (uint32_t*)(host.data() + o_f);
+    memcpy(host.data() + o_w, t_out, b_w);
+    size_t toff = 0, coff = 0, roff = 0;
     for (uint32_t d = 0; d < ndom; ++d) {
         score_ctx* c = doms[d];
-        EvoDev& v = evo[d];
-        v.t = d_t + toff;
+        EvoDev v{};
+        const uint32_t G = c->ndefg + c->nrxg;
+        v.t = (const double*)(blk + o_t) + toff;
         v.counts = c->d_log_counts;
         v.fin_defg = c->a.defg_cnt;
         v.fin_rxg = c->a.rxg_cnt;
-        v.cls = cls ? d_c + coff : nullptr;
-        v.ndefg = c->ndefg; v.nrxg = c->nrxg; v.nsnap = (uint32_t)c->log_info.size(); v.pad = 0;
+        v.ndefg = c->ndefg; v.nrxg = c->nrxg; v.nsnap = (uint32_t)c->log_info.size();
+        v.ngr = cls ? G : c->ndefg;
         v.tsimend = c->ph.t; v.nboxvol = (double)c->N;
-        for (const auto& info : c->log_info) times.push_back(info.t);
-        toff += c->log_info.size();
-        coff += (size_t)c->ndefg + c->nrxg;
+        if (cls) {  // grains by class, in grain order within a class
+            v.order = (const uint32_t*)(blk + o_o) + coff;
+            v.first = (const uint32_t*)(blk + o_f) + (size_t)d * (nc + 1);
+            uint32_t* f = first + (size_t)d * (nc + 1);
+            for (uint32_t k = 0; k <= nc; ++k) f[k] = 0;
+            for (uint32_t g = 0; g < G; ++g) f[cls[coff + g] + 1]++;
+            for (uint32_t k = 0; k < nc; ++k) f[k + 1] += f[k];
+            uint32_t at[kMaxClasses];
+            for (uint32_t k = 0; k < nc; ++k) at[k] = f[k];
+            for (uint32_t g = 0; g < G; ++g) order[coff + at[cls[coff + g]]++] = g;
+        }
+        v.rows = (double2*)(blk + sent) + roff;
+        for (const auto& info : c->log_info) times[toff++] = info.t;
+        coff += G;
+        roff += ((size_t)v.nsnap + 2) * v.ngr;
+        evo[d] = v;
     }
     cudaStream_t st = doms[0]->stream;
-    e = cudaMemcpyAsync(d_evo, evo.data(), b_evo, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && b_t) e = cudaMemcpyAsync(d_t, times.data(), b_t, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_w, t_out, b_w, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && cls) e = cudaMemcpyAsync(d_c, cls, b_c, cudaMemcpyHostToDevice, st);
+    cudaError_t e = cudaMemcpyAsync(blk, host.data(), sent, cudaMemcpyHostToDevice, st);
+    double* const d_pd = (double*)(blk + o_pd);
+    double* const d_out = (double*)(blk + o_out);
     if (e == cudaSuccess) {
-        const uint32_t nt = ndom * nslots;
-        if (cls) k_rediscr_texture<<<(nt + 127) / 128, 128, 0, st>>>(d_evo, ndom, d_w, nslots, nclass, d_pd);
-        else k_rediscr_kinetics<<<(nt + 127) / 128, 128, 0, st>>>(d_evo, ndom, d_w, nslots, d_pd);
+        const EvoDev* d_evo = (const EvoDev*)blk;
+        k_rediscr_rows<<<dim3((unsigned)((maxgr + 255) / 256), ndom), 256, 0, st>>>(d_evo);
+        k_rediscr_sum<<<dim3((nslots + 31) / 32, nc, ndom), 32, 0, st>>>(d_evo, (const double*)(blk + o_w), nslots, nc, cls ? 0 : 1, d_pd);
         k_rediscr_ensemble<<<(m + 127) / 128, 128, 0, st>>>(d_pd, ndom, m, d_out);
-        doms[0]->launches += 2;
+        doms[0]->launches += 3;
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, b_out, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(blk);
     if (e != cudaSuccess) { err = std::string("post-processing: ") + cudaGetErrorString(e); return SCORE_ERR_CUDA; }
     return SCORE_OK;
 }
