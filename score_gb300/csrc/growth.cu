@@ -2638,12 +2638,17 @@ int score_percolation_analyze(score_ctx* c, int mode, score_perc_result* out, ui
     if (!c) return SCORE_ERR_ARG;
     if (!c->loaded) return c->fail(SCORE_ERR_STATE, "no domain loaded");
     cudaSetDevice(c->device);
-    // the analysis reads the grid in linear order: a copy in the attempt-mask array (free between steps)
-    k_unbrick<<<blocks_for(c->ncells, c->sms, 16), kBlock, 0, c->stream>>>(c->a, c->a.grid, c->a.amask);
-    c->launches++;
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return c->cuda_fail(e, "percolation grid");
-    return percolation_analyze(c->a.amask, c->nx, c->ny, c->nz, c->ndefg, mode, c->stream, c->sms, out, sizes, sizes_cap, labels, c->err);
+    // the full-cell arrays (N words each) are free between steps
+    if (!c->stage(percolation_scratch(c->nx, c->ny, c->nz))) return c->fail(SCORE_ERR_NOMEM, "percolation buffers");
+    PercBuffers b{};
+    b.grid = c->a.grid;
+    b.parent = c->a.tobm;
+    b.size = c->a.f[0].full;
+    b.label = c->a.amask;
+    b.compact = c->a.fcell;
+    b.scratch = c->d_stage;
+    c->launches += 7 + (labels ? 1 : 0);
+    return percolation_analyze(b, c->a.gbx, c->a.gby, c->nx, c->ny, c->nz, c->ndefg, mode, c->stream, c->sms, out, sizes, sizes_cap, labels, c->err);
 }
 
 int score_get_timing(score_ctx* c, score_timing* out) {
