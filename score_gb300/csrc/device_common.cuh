@@ -18,7 +18,7 @@ constexpr unsigned long long kPtabTag = 0xFFFE000000000000ull;      // | m: requ
 constexpr unsigned long long kMissVoid = 0xFFFFFFFFFFFFFFFFull;     // miss slot lost a race: no request
 
 // error flags (DevState::err)
-constexpr uint32_t kErrTimeout = 1u << 0;    // kept for the status code; no kernel waits on another
+constexpr uint32_t kErrTimeout = 1u << 0;    // a block gave up waiting for its group (fused steps)
 constexpr uint32_t kErrCapacity = 1u << 1;
 constexpr uint32_t kErrBorderRef = 1u << 2;
 constexpr uint32_t kErrKeyLimit = 1u << 3;
@@ -62,21 +62,34 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 #define SCORE_STENCIL_DX {-1, 0, 1, -1, 1, -1, 0, 1, -1, 0, 1, -1, 0, 1, -1, 0, 1, -1, 0, 1, -1, 0, 1, -1, 0, 1}
 #define SCORE_STENCIL_DY {-1, -1, -1, 0, 0, 1, 1, 1, 1, 1, 1, -1, -1, -1, 0, 0, 0, -1, -1, -1, 0, 0, 0, 1, 1, 1}
 #define SCORE_STENCIL_DZ {0, 0, 0, 0, 0, 0, 0, 0, -1, -1, -1, -1, -1, -1, -1, -1, -1, 1, 1, 1, 1, 1, 1, 1, 1, 1}
-__constant__ int8_t c_dx[26] = SCORE_STENCIL_DX;
-__constant__ int8_t c_dy[26] = SCORE_STENCIL_DY;
-__constant__ int8_t c_dz[26] = SCORE_STENCIL_DZ;
-// the same offsets for host code (linear neighbour offsets of interior cells)
 constexpr int8_t kStencilDx[26] = SCORE_STENCIL_DX;
 constexpr int8_t kStencilDy[26] = SCORE_STENCIL_DY;
 constexpr int8_t kStencilDz[26] = SCORE_STENCIL_DZ;
-__constant__ uint8_t c_code[26] = {16, 15, 14, 13, 12, 11, 10, 9, 19, 18, 17, 25, 24, 23, 22, 21, 20, 8, 7, 6, 5, 4, 3, 2, 1, 0};
-__constant__ uint8_t c_cls[26] = {2, 1, 2, 1, 1, 2, 1, 2, 3, 2, 3, 3, 2, 3, 2, 1, 2, 3, 2, 3, 2, 1, 2, 3, 2, 3};
-// velocity shape factor indexed by infector code (calcGrowthStepInside, SCORE_Kernel.cpp:4053-4055); 26 = nucleus
-__constant__ double c_sf[27] = {0.6494, 0.7957, 0.6494, 0.7957, 1.0000, 0.7957, 0.6494, 0.7957, 0.6494,
-                                0.7957, 1.0000, 0.7957, 1.0000, 1.0000, 0.7957, 1.0000, 0.7957,
-                                0.6494, 0.7957, 0.6494, 0.7957, 1.0000, 0.7957, 0.6494, 0.7957, 0.6494, 1.0};
-__constant__ float c_sf32[27] = {0.6494f, 0.7957f, 0.6494f, 0.7957f, 1.0000f, 0.7957f, 0.6494f, 0.7957f, 0.6494f,
-                                 0.7957f, 1.0000f, 0.7957f, 1.0000f, 1.0000f, 0.7957f, 1.0000f, 0.7957f,
-                                 0.6494f, 0.7957f, 0.6494f, 0.7957f, 1.0000f, 0.7957f, 0.6494f, 0.7957f, 0.6494f, 1.0f};
+// A direction in one word: dx + 1 | (dy + 1) << 2 | (dz + 1) << 4 | overshoot class << 6 | infector code << 8.  Kernels keep
+// the 26 words in shared memory: lanes of a warp that look at different directions make a constant load
+// one pass a direction (with seven such loads a new cell a recovering 384^3 front took 131.5 ms, without 129.0; a
+// 16-domain batch 59.3 and 58.4).
+constexpr uint8_t kCode[26] = {16, 15, 14, 13, 12, 11, 10, 9, 19, 18, 17, 25, 24, 23, 22, 21, 20, 8, 7, 6, 5, 4, 3, 2, 1, 0};
+constexpr uint32_t dir_word(int d) {
+    const int dx = kStencilDx[d], dy = kStencilDy[d], dz = kStencilDz[d];
+    return (uint32_t)(dx + 1) | (uint32_t)(dy + 1) << 2 | (uint32_t)(dz + 1) << 4 | (uint32_t)((dx != 0) + (dy != 0) + (dz != 0)) << 6 |
+           (uint32_t)kCode[d] << 8;
+}
+struct DirWords { uint32_t v[26]; };
+constexpr DirWords dir_words() {
+    DirWords t{};
+    for (int d = 0; d < 26; ++d) t.v[d] = dir_word(d);
+    return t;
+}
+__constant__ DirWords c_dir = dir_words();
+__device__ __forceinline__ uint32_t dir_class(uint32_t w) { return (w >> 6) & 3u; }
+__device__ __forceinline__ uint32_t dir_code(uint32_t w) { return w >> 8; }
+// velocity shape factor of an infector code (calcGrowthStepInside, SCORE_Kernel.cpp:4053-4055): 1 of a face neighbour
+// and a nucleus (26), .7957 of an edge, .6494 of a corner neighbour; by selects, as codes differ from lane to lane
+__device__ __forceinline__ double shape_factor(uint32_t code) {
+    constexpr uint32_t kFace = 1u << 4 | 1u << 10 | 1u << 12 | 1u << 13 | 1u << 15 | 1u << 21 | 1u << 26;
+    constexpr uint32_t kCorner = 1u << 0 | 1u << 2 | 1u << 6 | 1u << 8 | 1u << 17 | 1u << 19 | 1u << 23 | 1u << 25;
+    return (kFace >> code) & 1u ? 1.0 : (kCorner >> code) & 1u ? 0.6494 : 0.7957;
+}
 
 }  // namespace score

@@ -113,7 +113,7 @@ struct FuseShared {
     uint32_t off[kFuseMaxLocal + 1];   // first record of each of the block's tiles
     uint32_t w1[kFuseWarps], w2[kFuseWarps];
     uint32_t t0[2], tot[2];            // counts before the Border list's tiles, and in all
-    uint32_t dir[26];                  // directions for moore_word
+    uint32_t dir[26];                  // dir_word of the directions
     uint32_t word, ok;
 };
 
@@ -235,9 +235,9 @@ __device__ __forceinline__ bool moore_of(const DomainArgs& a, int L, uint32_t ce
     m.near = !(x > 1 && x < nx - 2 && y > 1 && y < ny - 2 && z > 1 && z < nz - 2);
     return true;
 }
-// the neighbour in a direction packed as (dx + 1) | (dy + 1) << 2 | (dz + 1) << 4; false where z is open
+// the neighbour in a direction (dir_word); false where z is open
 __device__ __forceinline__ bool moore_word(const Moore& m, uint32_t dir, uint32_t& t, bool& interior) {
-    const uint32_t i = dir & 3u, j = (dir >> 2) & 3u, k = dir >> 4;
+    const uint32_t i = dir & 3u, j = (dir >> 2) & 3u, k = (dir >> 4) & 3u;
     t = (i == 0 ? m.X[0] : i == 1 ? m.X[1] : m.X[2]) + (j == 0 ? m.Y[0] : j == 1 ? m.Y[1] : m.Y[2]) + (k == 0 ? m.Z[0] : k == 1 ? m.Z[1] : m.Z[2]);
     interior = ((m.inner >> i) & (m.inner >> (3u + j)) & (m.inner >> (6u + k)) & 1u) != 0u;
     return (m.open >> k) & 1u;
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
     uint32_t n0 = st->next_never[0], n1 = st->next_never[1];
     uint32_t seq = map.seq[dom] & kCmdSeqMask, arrived = 0;
     if (threadIdx.x < 26)
-        sh.dir[threadIdx.x] = (uint32_t)(c_dx[threadIdx.x] + 1) | ((uint32_t)(c_dy[threadIdx.x] + 1) << 2) | ((uint32_t)(c_dz[threadIdx.x] + 1) << 4);
+        sh.dir[threadIdx.x] = c_dir.v[threadIdx.x];
     for (;;) {
         // ---- the host's word for step `seq`
         if (first) {
@@ -915,14 +915,14 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
                     decode(cst, sc & 0x7FFFFFFFu, x, y, z);
                     uint32_t tgt;
                     bool inter;
-                    target_of(cst, (int)(sc >> 31), x, y, z, d, tgt, inter);
+                    target_of(cst, (int)(sc >> 31), x, y, z, sh.dir[d], tgt, inter);
                     const uint32_t gt = cst.grid[tgt];
                     const DFront& dst = a.f[D];
                     const uint32_t nrec = D ? nrec1 : nrec0;
                     const uint32_t ns = r < nrec ? dst.recyc[r] : (D ? n1 : n0) + (r - nrec);
                     if (ns >= dst.cap) { atomicOr(&st->err, kErrCapacity); continue; }
                     if (D == 1 && cst.border_policy == 0 && r >= nrec && ns >= cst.border_ref_cap) atomicOr(&st->err, kErrBorderRef);
-                    new_cell<FP32>(a, dst, ns, tgt, gt, sh.c_rs[t], sh.c_over[t], d, pmax, ntag);
+                    new_cell<FP32>(a, dst, ns, tgt, gt, sh.c_rs[t], sh.c_over[t], sh.dir[d], pmax, ntag);
                 }
             }
             if (fc.gk && fc.gold == fc.gk) {  // the deformed grain's last cells

@@ -164,11 +164,11 @@ __device__ __forceinline__ uint32_t linear_of(const DomainArgs& a, int x, int y,
     return (uint32_t)x + a.nx * ((uint32_t)y + a.ny * (uint32_t)z);
 }
 
-// Target of attempt d from (x,y,z) of a cell of list L.  Inside cells are strictly
+// Target of an attempt in a direction (dir_word) from (x,y,z) of a cell of list L.  Inside cells are strictly
 // interior so their neighbours need no wrap; Border cells wrap x,y periodically and
 // drop z (reference) or wrap z (periodic build option).  false = attempt dropped.
-__device__ __forceinline__ bool target_of(const DomainArgs& a, int L, int x, int y, int z, int d, uint32_t& t, bool& interior) {
-    int tx = x + c_dx[d], ty = y + c_dy[d], tz = z + c_dz[d];
+__device__ __forceinline__ bool target_of(const DomainArgs& a, int L, int x, int y, int z, uint32_t dw, uint32_t& t, bool& interior) {
+    int tx = x + (int)(dw & 3u) - 1, ty = y + (int)((dw >> 2) & 3u) - 1, tz = z + (int)((dw >> 4) & 3u) - 1;
     if (L == 1) {
         if (tx < 0) tx += (int)a.nx;
         if (tx >= (int)a.nx) tx -= (int)a.nx;
@@ -200,7 +200,7 @@ __device__ __forceinline__ double velocity_from_force(double m, double p, int co
     // p > 5e-16 by integers (an FP64 compare takes the FP64 pipe, 1/64 rate); a NaN is not above it
     const long long b = __double_as_longlong(p);
     if (!(b > __double_as_longlong(5.0e-16) && b <= 0x7FF0000000000000ll)) return -1.0;
-    return __dmul_rn(__dmul_rn(m, p), c_sf[code]);
+    return __dmul_rn(__dmul_rn(m, p), shape_factor((uint32_t)code));
 }
 __device__ __forceinline__ double velocity_from_mobility(const DomainArgs& a, double m, uint32_t defg, int code) {
     return velocity_from_force(m, a.pforce[defg], code);
@@ -1298,7 +1298,7 @@ __device__ __forceinline__ uint32_t claim_plane(const DomainArgs& a, int x, int 
     for (int k = 0; k < HI - LO; ++k) {
         gv[k] = 0xFFFFFFFFu;
         bool inter;
-        if (target_of(a, 1, x, y, z, LO + k, tg[k], inter)) gv[k] = a.grid[tg[k]];
+        if (target_of(a, 1, x, y, z, c_dir.v[LO + k], tg[k], inter)) gv[k] = a.grid[tg[k]];
     }
     uint32_t mask = 0;
 #pragma unroll
@@ -1693,7 +1693,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_resolve(int base, int ndom) {
                     if ((mask >> d) & 1u) {
                         uint32_t t;
                         bool inter;
-                        target_of(a, L, x, y, z, d, t, inter);
+                        target_of(a, L, x, y, z, c_dir.v[d], t, inter);
                         cl[d] = a.claim[t];
                         if (inter) inter_m |= 1u << d;
                     }
@@ -1763,13 +1763,13 @@ __device__ __forceinline__ void count_full(const DomainArgs& a, bool has, uint32
 }
 
 // A newly infected cell tgt (deformed grain gt until now) takes slot ns of list `dst`: overshoot `over` of the
-// full cell scaled by the direction's class, infector code of direction d, rx grain rs, and its mobility
+// full cell scaled by the direction's class, infector code of the direction (dir_word), rx grain rs, and its mobility
 // weight and cached velocity factor (or a tag for the host's answer).
 template <bool FP32>
 __device__ __forceinline__ void new_cell(const DomainArgs& a, const DFront& dst, uint32_t ns, uint32_t tgt, uint32_t gt, uint32_t rs,
-                                         double over, int d, double& pmax, uint32_t& ntag) {
+                                         double over, uint32_t dw, double& pmax, uint32_t& ntag) {
     const double pf = a.pforce[gt];  // in flight together with the weight's load
-    const int cls = c_cls[d];
+    const uint32_t cls = dir_class(dw), code = dir_code(dw);
     if (!FP32) {
         const double fac = cls == 1 ? 0.0682 : (cls == 2 ? 0.0542 : 0.0484);
         ((double*)dst.fill)[ns] = __dmul_rn(over, fac);
@@ -1789,7 +1789,7 @@ __device__ __forceinline__ void new_cell(const DomainArgs& a, const DFront& dst,
     if (lookup_p(a, rs, gt, P, tag)) {
         const double mo = mobility(a, P);
         dst.mob[ns] = mo;
-        const double v = velocity_from_force(mo, pf, c_code[d]);
+        const double v = velocity_from_force(mo, pf, (int)code);
         if (!FP32) {
             // the increment with this step's dt: valid next step unless dt changes, when
             // k_grow_fill recomputes every increment from vel anyway
@@ -1798,13 +1798,13 @@ __device__ __forceinline__ void new_cell(const DomainArgs& a, const DFront& dst,
         } else {
             ((float*)dst.vel)[ns] = (float)v;
         }
-        dst.dir[ns] = c_code[d];
+        dst.dir[ns] = (uint8_t)code;
         if (P > pmax) pmax = P;
     } else {
         // vel holds the answer tag until the next k_grow_fill
         if (!FP32) ((unsigned long long*)dst.vel)[ns] = tag;
         else ((uint32_t*)dst.vel)[ns] = tag;
-        dst.dir[ns] = c_code[d] | kStale | kPend;
+        dst.dir[ns] = (uint8_t)(code | kStale | kPend);
         ++ntag;
     }
 }
@@ -1816,6 +1816,8 @@ __global__ void __launch_bounds__(kBlock, ONE ? 4 : 3) k_commit(int base, int nd
     // per full cell of the tile: win masks, first ranks, cell (| Border list << 31), grain, overshoot
     __shared__ uint32_t s_off[kBlock + 1], s_win[kBlock], s_tob[kBlock], s_rA[kBlock], s_rB[kBlock], s_cell[kBlock], s_rsrc[kBlock];
     __shared__ double s_over[kBlock];
+    __shared__ uint32_t s_dir[26];
+    if (threadIdx.x < 26) s_dir[threadIdx.x] = c_dir.v[threadIdx.x];  // seen after the tiles' first barrier
     const uint32_t total = ONE ? commit_tiles(c_args[base])
                                : seg_prefix(s_pre, ndom, [&](int s) { return commit_tiles(c_args[base + (s)]); });
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1906,14 +1908,14 @@ __global__ void __launch_bounds__(kBlock, ONE ? 4 : 3) k_commit(int base, int nd
             decode(a, sc & 0x7FFFFFFFu, x, y, z);
             uint32_t tgt;
             bool inter;
-            target_of(a, Ls, x, y, z, d, tgt, inter);
+            target_of(a, Ls, x, y, z, s_dir[d], tgt, inter);
             const uint32_t gt = a.grid[tgt];  // in flight together with the slot's load
             const DFront& dst = a.f[D];
             const uint32_t nrec = a.st->nrec[D];
             const uint32_t ns = r < nrec ? dst.recyc[r] : a.st->next_never[D] + (r - nrec);
             if (ns >= dst.cap) { atomicOr(&a.st->err, kErrCapacity); continue; }
             if (D == 1 && a.border_policy == 0 && r >= nrec && ns >= a.border_ref_cap) atomicOr(&a.st->err, kErrBorderRef);
-            new_cell<FP32>(a, dst, ns, tgt, gt, s_rsrc[t], s_over[t], d, pmax, ntag);
+            new_cell<FP32>(a, dst, ns, tgt, gt, s_rsrc[t], s_over[t], s_dir[d], pmax, ntag);
         }
         if (f < F) {
             // the full cell is now recrystallized
