@@ -195,54 +195,6 @@ __device__ __forceinline__ void tile_scan(FuseShared& sh, const uint2* cnt, uint
     __syncthreads();
 }
 
-// The grid words of a cell's 26 neighbours as sums of three terms: in bricks, a word is
-// 8 ((z/2) gbxy + (y/2) gbx + x/2) + 4 (z%2) + 2 (y%2) + x%2, so each axis gives a term for -1, 0 and +1 with its
-// wrap done once.  Border cells wrap in x and y and drop z (reference) or wrap it (periodic option); Inside
-// cells are strictly interior.
-struct Moore {
-    uint32_t X[3], Y[3], Z[3];
-    uint32_t open;     // bit k: offset k - 1 along z exists
-    uint32_t inner;    // bits 0-2 x, 3-5 y, 6-8 z: the offset's coordinate is not on a face
-    bool near;         // the cell lies on the second layer below a face: an Inside cell's infections go to the Border list
-};
-__device__ __forceinline__ bool moore_of(const DomainArgs& a, int L, uint32_t cell, Moore& m) {
-    int x, y, z;
-    decode(a, cell, x, y, z);
-    const int nx = (int)a.nx, ny = (int)a.ny, nz = (int)a.nz;
-    if (L == 0 && !(x > 0 && y > 0 && z > 0 && x < nx - 1 && y < ny - 1 && z < nz - 1)) {
-        atomicOr(&a.st->err, kErrBounds);
-        return false;
-    }
-    m.open = 0u; m.inner = 0u;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        int tx = x + k - 1, ty = y + k - 1, tz = z + k - 1;
-        if (tx < 0) tx += nx;
-        if (tx >= nx) tx -= nx;
-        if (ty < 0) ty += ny;
-        if (ty >= ny) ty -= ny;
-        bool in = true;
-        if (tz < 0) { in = a.boundary != 0; tz += nz; }
-        if (tz >= nz) { in = a.boundary != 0; tz -= nz; }
-        m.X[k] = (((uint32_t)tx >> 1) << 3) | ((uint32_t)tx & 1u);
-        m.Y[k] = ((((uint32_t)ty >> 1) * a.gbx) << 3) | (((uint32_t)ty & 1u) << 1);
-        m.Z[k] = ((((uint32_t)tz >> 1) * a.gbxy) << 3) | (((uint32_t)tz & 1u) << 2);
-        m.open |= (in ? 1u : 0u) << k;
-        m.inner |= (tx > 0 && tx < nx - 1 ? 1u : 0u) << k;
-        m.inner |= (ty > 0 && ty < ny - 1 ? 8u : 0u) << k;
-        m.inner |= (tz > 0 && tz < nz - 1 ? 64u : 0u) << k;
-    }
-    m.near = !(x > 1 && x < nx - 2 && y > 1 && y < ny - 2 && z > 1 && z < nz - 2);
-    return true;
-}
-// the neighbour in a direction (dir_word); false where z is open
-__device__ __forceinline__ bool moore_word(const Moore& m, uint32_t dir, uint32_t& t, bool& interior) {
-    const uint32_t i = dir & 3u, j = (dir >> 2) & 3u, k = (dir >> 4) & 3u;
-    t = (i == 0 ? m.X[0] : i == 1 ? m.X[1] : m.X[2]) + (j == 0 ? m.Y[0] : j == 1 ? m.Y[1] : m.Y[2]) + (k == 0 ? m.Z[0] : k == 1 ? m.Z[1] : m.Z[2]);
-    interior = ((m.inner >> i) & (m.inner >> (3u + j)) & (m.inner >> (6u + k)) & 1u) != 0u;
-    return (m.open >> k) & 1u;
-}
-
 // overshoot of a full cell, for the cells it infects
 template <bool FP32>
 __device__ __forceinline__ double full_over(const DFront& fr, uint32_t slot) {
@@ -530,16 +482,7 @@ __device__ __forceinline__ void take_full(const DomainArgs& cst, const DomainArg
         if (!FP32) ((double*)fr.fill)[slot] = 0.0;
         else { ((float*)fr.fill)[slot] = 0.0f; fr.comp[slot] = 0.0f; }
     }
-    const uint32_t has = __ballot_sync(0xFFFFFFFFu, i < F);
-    if (!has) return;
-    const int lane = threadIdx.x & 31;
-    const uint32_t mr = __match_any_sync(0xFFFFFFFFu, i < F ? c.rs : 0xFFFFFFFFu) & has;
-    const uint32_t mg = __match_any_sync(0xFFFFFFFFu, i < F ? c.gs : 0xFFFFFFFFu) & has;
-    if (i < F && (__ffs(mr) - 1) == lane) atomicAdd(&cst.rxg_cnt[c.rs], (uint32_t)__popc(mr));
-    if (i < F && (__ffs(mg) - 1) == lane) {
-        c.gk = (uint32_t)__popc(mg);
-        c.gold = atomicSub(&cst.defg_cnt[c.gs], c.gk);
-    }
+    count_full(cst, i < F, c.rs, c.gs, c.gk, c.gold);
 }
 
 template <bool FP32, int ITEMS>
@@ -721,35 +664,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
                 uint32_t mask = 0;
                 if (i < F) {
                     const uint32_t ord = ((key & 0x7FFFFFFFu) + (key >> 31 ? n0 : 0u)) * 26u;
-                    int x, y, z;
-                    decode(cst, cell, x, y, z);
-                    if (x > 0 && y > 0 && z > 0 && x < (int)cst.nx - 1 && y < (int)cst.ny - 1 && z < (int)cst.nz - 1) {
-                        const int b = lane & 3;
-                        const uint32_t w0 = brick_word(cst, x, y, z, b), w1 = brick_word(cst, x, y, z, b + 4);
-                        Brick r0, r1;
-                        load_brick(cst.grid + w0, r0);
-                        load_brick(cst.grid + w1, r1);
-                        mask = claim_brick(cst, x, y, z, b, w0, r0, ord) | claim_brick(cst, x, y, z, b + 4, w1, r1, ord);
-                    } else {
-                        Moore mo;
-                        if (moore_of(cst, (int)(key >> 31), cell, mo)) {
-                            uint32_t tg[7], gv[7];
-#pragma unroll
-                            for (int k = 0; k < 7; ++k) {
-                                const uint32_t d = (uint32_t)(lane & 3) + 4u * (uint32_t)k;
-                                bool inter;
-                                gv[k] = 0xFFFFFFFFu;
-                                if (d < 26u && moore_word(mo, sh.dir[d], tg[k], inter)) gv[k] = cst.grid[tg[k]];
-                            }
-#pragma unroll
-                            for (int k = 0; k < 7; ++k) {
-                                const uint32_t d = (uint32_t)(lane & 3) + 4u * (uint32_t)k;
-                                if (gv[k] >= cst.ndefg) continue;
-                                atomicMin(&cst.claim[tg[k]], ord + d);
-                                mask |= 1u << d;
-                            }
-                        }
-                    }
+                    mask = attempt_quarter(cst, (int)(key >> 31), cell, ord, lane & 3, sh.dir);
                 }
                 mask |= __shfl_xor_sync(0xFFFFFFFFu, mask, 1);
                 mask |= __shfl_xor_sync(0xFFFFFFFFu, mask, 2);
@@ -803,35 +718,8 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             uint32_t win = 0, tob = 0, key = 0;
             if (i < F) {
                 key = rec.key(i);
-                const uint32_t mask = rec.win(i);
-                Moore mo;
-                if (mask && moore_of(cst, (int)(key >> 31), rec.cell(i), mo)) {
-                    const uint32_t s = (key & 0x7FFFFFFFu) + (key >> 31 ? n0 : 0u);
-                    // the lane's share of the attempts made, their claims in flight together
-                    uint32_t m = mask & (0x01111111u << (lane & 3)), cl[7], at[7], inm = 0;
-#pragma unroll
-                    for (int k = 0; k < 7; ++k) {
-                        at[k] = 0xFFFFFFFFu; cl[k] = kClaimFree;
-                        if (m) {
-                            at[k] = (uint32_t)(__ffs(m) - 1);
-                            m &= m - 1u;
-                            uint32_t t;
-                            bool inter;
-                            moore_word(mo, sh.dir[at[k]], t, inter);
-                            cl[k] = cst.claim[t];
-                            inm |= (inter ? 1u : 0u) << k;
-                        }
-                    }
-#pragma unroll
-                    for (int k = 0; k < 7; ++k) {
-                        if (at[k] < 26u && cl[k] == s * 26u + at[k]) {
-                            win |= 1u << at[k];
-                            // Inside full cells near a face infect into the Border list (SCORE_Kernel.cpp:4606-4609);
-                            // Border full cells send strictly interior targets to the Inside list (:4387)
-                            if (key >> 31 ? !((inm >> k) & 1u) : mo.near) tob |= 1u << at[k];
-                        }
-                    }
-                }
+                const uint32_t s = (key & 0x7FFFFFFFu) + (key >> 31 ? n0 : 0u);
+                win_quarter(cst, (int)(key >> 31), rec.cell(i), rec.win(i), s * 26u, lane & 3, sh.dir, win, tob);
             }
             win |= __shfl_xor_sync(0xFFFFFFFFu, win, 1);
             tob |= __shfl_xor_sync(0xFFFFFFFFu, tob, 1);

@@ -567,7 +567,7 @@ void score_ctx::release_domain() {
 struct TuneCfg {
     int items = 8;          // grow tile = kBlock * items slots
     int fill_bpsm = 16;     // k_grow_fill blocks per SM
-    int claim_bpsm = 2;     // k_claim blocks per SM (autotuner's choice on the 512^3 workload)
+    int claim_bpsm = 4;     // k_claim blocks per SM: what fits at 64 registers
     int commit_bpsm = 8;    // k_resolve / k_commit blocks per SM (same)
     int spec_pct = 30;      // every slot's data loaded with its infector byte up to this INACTIVE share [%]
     int timing_every = 8;   // phase events on every k-th step of a run (0 never): each event costs

@@ -1289,26 +1289,52 @@ __device__ __forceinline__ void scan_pairs_block(uint32_t* cnt, uint32_t ntiles,
 }
 
 // ------------------------------------------------------------------ K2 claim
-// Attempts LO..HI-1 of one Border cell: the grid loads are all issued before the atomics
-// (claims are a min, so the order of the atomics does not matter); targets wrap through target_of.
-template <int LO, int HI>
-__device__ __forceinline__ uint32_t claim_plane(const DomainArgs& a, int x, int y, int z, uint32_t f) {
-    uint32_t tg[HI - LO], gv[HI - LO];
-#pragma unroll
-    for (int k = 0; k < HI - LO; ++k) {
-        gv[k] = 0xFFFFFFFFu;
-        bool inter;
-        if (target_of(a, 1, x, y, z, c_dir.v[LO + k], tg[k], inter)) gv[k] = a.grid[tg[k]];
+// The grid words of a cell's 26 neighbours as sums of three terms: in bricks, a word is
+// 8 ((z/2) gbxy + (y/2) gbx + x/2) + 4 (z%2) + 2 (y%2) + x%2, so each axis gives a term for -1, 0 and +1 with its
+// wrap done once.  Border cells wrap in x and y and drop z (reference) or wrap it (periodic option); Inside
+// cells are strictly interior.
+struct Moore {
+    uint32_t X[3], Y[3], Z[3];
+    uint32_t open;     // bit k: offset k - 1 along z exists
+    uint32_t inner;    // bits 0-2 x, 3-5 y, 6-8 z: the offset's coordinate is not on a face
+    bool near;         // the cell lies on the second layer below a face: an Inside cell's infections go to the Border list
+};
+__device__ __forceinline__ bool moore_of(const DomainArgs& a, int L, uint32_t cell, Moore& m) {
+    int x, y, z;
+    decode(a, cell, x, y, z);
+    const int nx = (int)a.nx, ny = (int)a.ny, nz = (int)a.nz;
+    if (L == 0 && !(x > 0 && y > 0 && z > 0 && x < nx - 1 && y < ny - 1 && z < nz - 1)) {
+        atomicOr(&a.st->err, kErrBounds);
+        return false;
     }
-    uint32_t mask = 0;
+    m.open = 0u; m.inner = 0u;
 #pragma unroll
-    for (int k = 0; k < HI - LO; ++k) {
-        if (gv[k] < a.ndefg) {
-            atomicMin(&a.claim[tg[k]], f * 26u + (uint32_t)(LO + k));
-            mask |= 1u << (LO + k);
-        }
+    for (int k = 0; k < 3; ++k) {
+        int tx = x + k - 1, ty = y + k - 1, tz = z + k - 1;
+        if (tx < 0) tx += nx;
+        if (tx >= nx) tx -= nx;
+        if (ty < 0) ty += ny;
+        if (ty >= ny) ty -= ny;
+        bool in = true;
+        if (tz < 0) { in = a.boundary != 0; tz += nz; }
+        if (tz >= nz) { in = a.boundary != 0; tz -= nz; }
+        m.X[k] = (((uint32_t)tx >> 1) << 3) | ((uint32_t)tx & 1u);
+        m.Y[k] = ((((uint32_t)ty >> 1) * a.gbx) << 3) | (((uint32_t)ty & 1u) << 1);
+        m.Z[k] = ((((uint32_t)tz >> 1) * a.gbxy) << 3) | (((uint32_t)tz & 1u) << 2);
+        m.open |= (in ? 1u : 0u) << k;
+        m.inner |= (tx > 0 && tx < nx - 1 ? 1u : 0u) << k;
+        m.inner |= (ty > 0 && ty < ny - 1 ? 8u : 0u) << k;
+        m.inner |= (tz > 0 && tz < nz - 1 ? 64u : 0u) << k;
     }
-    return mask;
+    m.near = !(x > 1 && x < nx - 2 && y > 1 && y < ny - 2 && z > 1 && z < nz - 2);
+    return true;
+}
+// the neighbour in a direction (dir_word); false where z is open
+__device__ __forceinline__ bool moore_word(const Moore& m, uint32_t dir, uint32_t& t, bool& interior) {
+    const uint32_t i = dir & 3u, j = (dir >> 2) & 3u, k = (dir >> 4) & 3u;
+    t = (i == 0 ? m.X[0] : i == 1 ? m.X[1] : m.X[2]) + (j == 0 ? m.Y[0] : j == 1 ? m.Y[1] : m.Y[2]) + (k == 0 ? m.Z[0] : k == 1 ? m.Z[1] : m.Z[2]);
+    interior = ((m.inner >> i) & (m.inner >> (3u + j)) & (m.inner >> (6u + k)) & 1u) != 0u;
+    return (m.open >> k) & 1u;
 }
 
 // One of the 8 bricks around an interior cell (x, y, z), the 32 bytes by one load: the lower (0) or upper (1) brick of
@@ -1350,6 +1376,69 @@ __device__ __forceinline__ uint32_t claim_brick(const DomainArgs& a, int x, int 
     return mask;
 }
 
+// One lane's share (`sub` of four) of a full cell's 26 infection attempts, ordinals key + direction: an interior cell's 8
+// bricks two a lane, a face cell's directions 6 or 7 a lane; s_dir: the direction words.  Returns their bits.
+__device__ __forceinline__ uint32_t attempt_quarter(const DomainArgs& a, int L, uint32_t cell, uint32_t key, int sub, const uint32_t* s_dir) {
+    uint32_t mask = 0;
+    int x, y, z;
+    decode(a, cell, x, y, z);
+    if (x > 0 && y > 0 && z > 0 && x < (int)a.nx - 1 && y < (int)a.ny - 1 && z < (int)a.nz - 1) {
+        const uint32_t w0 = brick_word(a, x, y, z, sub), w1 = brick_word(a, x, y, z, sub + 4);
+        Brick r0, r1;
+        load_brick(a.grid + w0, r0);
+        load_brick(a.grid + w1, r1);
+        return claim_brick(a, x, y, z, sub, w0, r0, key) | claim_brick(a, x, y, z, sub + 4, w1, r1, key);
+    }
+    Moore mo;
+    if (!moore_of(a, L, cell, mo)) return 0u;
+    uint32_t tg[7], gv[7];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        const uint32_t d = (uint32_t)sub + 4u * (uint32_t)k;
+        bool inter;
+        gv[k] = 0xFFFFFFFFu;
+        if (d < 26u && moore_word(mo, s_dir[d], tg[k], inter)) gv[k] = a.grid[tg[k]];
+    }
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        const uint32_t d = (uint32_t)sub + 4u * (uint32_t)k;
+        if (gv[k] >= a.ndefg) continue;
+        atomicMin(&a.claim[tg[k]], key + d);
+        mask |= 1u << d;
+    }
+    return mask;
+}
+// The lane's share of the attempts `mask` of the cell that won: the claim of the target holds the attempt's ordinal.
+// tob: those whose new cell goes to the Border list; Inside full cells near a face infect into it
+// (SCORE_Kernel.cpp:4606-4609), Border full cells send strictly interior targets to the Inside list (:4387).
+__device__ __forceinline__ void win_quarter(const DomainArgs& a, int L, uint32_t cell, uint32_t mask, uint32_t key, int sub, const uint32_t* s_dir,
+                                            uint32_t& win, uint32_t& tob) {
+    Moore mo;
+    if (!mask || !moore_of(a, L, cell, mo)) return;
+    // the claims of the lane's attempts in flight together
+    uint32_t m = mask & (0x01111111u << sub), cl[7], at[7], inm = 0;
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        at[k] = 0xFFFFFFFFu; cl[k] = kClaimFree;
+        if (m) {
+            at[k] = (uint32_t)(__ffs(m) - 1);
+            m &= m - 1u;
+            uint32_t t;
+            bool inter;
+            moore_word(mo, s_dir[at[k]], t, inter);
+            cl[k] = a.claim[t];
+            inm |= (inter ? 1u : 0u) << k;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        if (at[k] < 26u && cl[k] == key + at[k]) {
+            win |= 1u << at[k];
+            if (L ? !((inm >> k) & 1u) : mo.near) tob |= 1u << at[k];
+        }
+    }
+}
+
 // full cells of a domain this step (Inside list first); 0 when the 32-bit attempt
 // ordinal 26 f + d could overflow (flagged)
 __device__ __forceinline__ uint32_t full_cells(const DomainArgs& a) {
@@ -1358,9 +1447,13 @@ __device__ __forceinline__ uint32_t full_cells(const DomainArgs& a) {
     return 26ull * F >= 0xFFFFFFFFull ? 0u : F;
 }
 
+// Bound by the chain list -> position -> bricks -> claims, not by its bytes (25 % of DRAM): four lanes a full cell, and the
+// next cell's position in flight meanwhile.  A thread a cell, its 8 bricks in 128 registers at two blocks a SM: 19.1 ms
+// of a 512^3 run, now 16.8; 13.0 and 10.6 of a 384^3 front of sheets; 18.0 and 15.3 of a 16-domain batch.
 template <bool ONE>
-__global__ void __launch_bounds__(kBlock, 2) k_claim(int base, int ndom) {
-    __shared__ uint32_t s_pre[kMaxSegs + 1], s_cnt[kMaxSegs];
+__global__ void __launch_bounds__(kBlock, 4) k_claim(int base, int ndom) {
+    __shared__ uint32_t s_pre[kMaxSegs + 1], s_cnt[kMaxSegs], s_dir[26];
+    if (threadIdx.x < 26) s_dir[threadIdx.x] = c_dir.v[threadIdx.x];
     auto count = [&](int s) {
         const DomainArgs& a = c_args[base + (s)];
         if (a.active && 26ull * (a.st->nfull[0] + a.st->nfull[1]) >= 0xFFFFFFFFull) atomicOr(&a.st->err, kErrKeyLimit);
@@ -1369,47 +1462,43 @@ __global__ void __launch_bounds__(kBlock, 2) k_claim(int base, int ndom) {
     uint32_t total;
     if (ONE) {
         total = count(0);
+        __syncthreads();
     } else {
         total = seg_prefix(s_pre, ndom, [&](int s) {
             s_cnt[s] = count(s);
             return warp_pad(s_cnt[s]);
         });
     }
-    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < total; u += gridDim.x * blockDim.x) {
-        const int s = ONE ? 0 : seg_find(s_pre, ndom, u);
-        const DomainArgs& a = c_args[base + (s)];
-        const uint32_t f = ONE ? u : u - s_pre[s];
-        if (!ONE && f >= s_cnt[s]) continue;
+    const int lane = threadIdx.x & 31, sub = lane & 3;
+    // cell u of the launch: domain, full-cell number, list, position
+    struct At { uint32_t f, cell; int s, L; bool is; };
+    auto locate = [&](uint32_t u) {
+        At t{0u, 0u, 0, 0, false};
+        if (u >= total) return t;
+        t.s = ONE ? 0 : seg_find(s_pre, ndom, u);
+        t.f = ONE ? u : u - s_pre[t.s];
+        if (!ONE && t.f >= s_cnt[t.s]) return t;
+        const DomainArgs& a = c_args[base + t.s];
         const uint32_t F0 = a.st->nfull[0];
-        uint32_t mask;
-        if (f < F0) {
-            // an Inside cell (strictly interior, every list insertion checks it): its neighbourhood
-            // spans 8 bricks, one 32-byte load each, all in flight before the first claim (26 word loads a
-            // cell took 26 passes of the L1's tag stage a cell instead of 8)
-            const uint32_t cell = a.f[0].xyz[a.f[0].full[f]];
-            a.fcell[f] = cell;
-            int x, y, z;
-            decode(a, cell, x, y, z);
-            mask = 0;
-            if (x < 1 || y < 1 || z < 1 || x > (int)a.nx - 2 || y > (int)a.ny - 2 || z > (int)a.nz - 2) {
-                atomicOr(&a.st->err, kErrBounds);
-            } else {
-                Brick r[8];
-#pragma unroll
-                for (int b = 0; b < 8; ++b) load_brick(a.grid + brick_word(a, x, y, z, b), r[b]);
-#pragma unroll
-                for (int b = 0; b < 8; ++b) mask |= claim_brick(a, x, y, z, b, brick_word(a, x, y, z, b), r[b], f * 26u);
-            }
-        } else {
-            const uint32_t cell = a.f[1].xyz[a.f[1].full[f - F0]];
-            a.fcell[f] = cell;
-            int x, y, z;
-            decode(a, cell, x, y, z);
-            mask = claim_plane<0, 8>(a, x, y, z, f);
-            mask |= claim_plane<8, 17>(a, x, y, z, f);
-            mask |= claim_plane<17, 26>(a, x, y, z, f);
+        t.L = t.f < F0 ? 0 : 1;
+        t.cell = t.L ? a.f[1].xyz[a.f[1].full[t.f - F0]] : a.f[0].xyz[a.f[0].full[t.f]];
+        t.is = true;
+        return t;
+    };
+    const uint32_t step = gridDim.x * (kBlock / 4);
+    uint32_t u0 = (blockIdx.x * kWarps + (threadIdx.x >> 5)) * 8u;
+    At t = locate(u0 + (uint32_t)(lane >> 2));
+    for (; u0 < total; u0 += step) {
+        const At next = locate(u0 + step + (uint32_t)(lane >> 2));
+        const DomainArgs& a = c_args[base + t.s];
+        uint32_t mask = t.is ? attempt_quarter(a, t.L, t.cell, t.f * 26u, sub, s_dir) : 0u;
+        mask |= __shfl_xor_sync(0xFFFFFFFFu, mask, 1);
+        mask |= __shfl_xor_sync(0xFFFFFFFFu, mask, 2);
+        if (t.is && sub == 0) {
+            a.fcell[t.f] = t.cell;
+            a.amask[t.f] = mask;
         }
-        a.amask[f] = mask;
+        t = next;
     }
 }
 
@@ -1654,8 +1743,8 @@ __device__ __forceinline__ void step_end_block(const DomainArgs& a, uint32_t gro
 }
 
 // ------------------------------------------------------------------ K3 commit (+ finalize)
-// k_resolve: one thread per full cell, tiles of kBlock full cells: its attempts whose
-// claim holds the own ordinal won; writes the win mask, the mask of wins that go to
+// k_resolve: four lanes per full cell (a thread a cell: 12.6 ms for both kernels of a 120^3 domain, now
+// 11.7; large fronts the same), tiles of kBlock full cells: its attempts whose claim holds the own ordinal won; writes the win mask, the mask of wins that go to
 // the Border list, the tile's two win counts and adds them to its supertile.
 // k_commit: winners are ranked per destination list in full-cell then direction
 // order (tile prefix from the supertile and tile counts) and take recycled slots
@@ -1666,7 +1755,9 @@ __device__ __forceinline__ uint32_t commit_tiles(const DomainArgs& a) { return (
 template <bool ONE>
 __global__ void __launch_bounds__(kBlock, 4) k_resolve(int base, int ndom) {
     __shared__ uint32_t s_pre[kMaxSegs + 1];
-    __shared__ uint32_t s_a[kWarps], s_b[kWarps];
+    __shared__ uint32_t s_a[kWarps], s_b[kWarps], s_dir[26];
+    if (threadIdx.x < 26) s_dir[threadIdx.x] = c_dir.v[threadIdx.x];
+    __syncthreads();
     const uint32_t total = ONE ? commit_tiles(c_args[base])
                                : seg_prefix(s_pre, ndom, [&](int s) { return commit_tiles(c_args[base + (s)]); });
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1675,39 +1766,28 @@ __global__ void __launch_bounds__(kBlock, 4) k_resolve(int base, int ndom) {
         const DomainArgs& a = c_args[base + (s)];
         const uint32_t tile = ONE ? u : u - s_pre[s];
         const uint32_t F0 = a.st->nfull[0], F = F0 + a.st->nfull[1];
-        const uint32_t f = tile * kBlock + threadIdx.x;
-        uint32_t win = 0, tob = 0;
+        // a warp takes 32 full cells, 8 at a time, four lanes each; lane 4 j + i ends up with cell 8 i + j of them
+        const uint32_t f0 = tile * kBlock + (uint32_t)warp * 32u;
+        uint32_t mk[4], cell[4], win = 0, tob = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t f = f0 + 8u * (uint32_t)i + (uint32_t)(lane >> 2);
+            mk[i] = f < F ? a.amask[f] : 0u;
+            cell[i] = f < F ? a.fcell[f] : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t f = f0 + 8u * (uint32_t)i + (uint32_t)(lane >> 2);
+            uint32_t w = 0, b = 0;
+            win_quarter(a, f >= F0 ? 1 : 0, cell[i], mk[i], f * 26u, lane & 3, s_dir, w, b);
+            w |= __shfl_xor_sync(0xFFFFFFFFu, w, 1);
+            b |= __shfl_xor_sync(0xFFFFFFFFu, b, 1);
+            w |= __shfl_xor_sync(0xFFFFFFFFu, w, 2);
+            b |= __shfl_xor_sync(0xFFFFFFFFu, b, 2);
+            if ((lane & 3) == i) { win = w; tob = b; }
+        }
+        const uint32_t f = f0 + 8u * (uint32_t)(lane & 3) + (uint32_t)(lane >> 2);
         if (f < F) {
-            const uint32_t mask = a.amask[f];
-            if (mask) {
-                const int L = f >= F0 ? 1 : 0;
-                const uint32_t cell = a.fcell[f];
-                int x, y, z;
-                decode(a, cell, x, y, z);
-                const bool allB = (L == 0) && !(x > 1 && x < (int)a.nx - 2 && y > 1 && y < (int)a.ny - 2 && z > 1 && z < (int)a.nz - 2);
-                uint32_t cl[26];
-                uint32_t inter_m = 0;
-#pragma unroll
-                for (int d = 0; d < 26; ++d) {
-                    cl[d] = kClaimFree;
-                    if ((mask >> d) & 1u) {
-                        uint32_t t;
-                        bool inter;
-                        target_of(a, L, x, y, z, c_dir.v[d], t, inter);
-                        cl[d] = a.claim[t];
-                        if (inter) inter_m |= 1u << d;
-                    }
-                }
-#pragma unroll
-                for (int d = 0; d < 26; ++d) {
-                    if (cl[d] == f * 26u + (uint32_t)d) {
-                        win |= 1u << d;
-                        // Inside full cells near a face infect into the Border list (:4606-4609);
-                        // Border full cells send strictly interior targets to the Inside list (:4387)
-                        if (L == 0 ? allB : !((inter_m >> d) & 1u)) tob |= 1u << d;
-                    }
-                }
-            }
             a.amask[f] = win;
             a.tobm[f] = tob;
         }
@@ -1745,20 +1825,18 @@ __device__ __forceinline__ void flush_new(const DomainArgs& a, double pmax, uint
 }
 
 // per-grain cell counts of a warp's recrystallized cells (rx grain rs, deformed grain gs): one atomic per
-// grain and warp (full cells of one grain tend to finish together); every lane takes part
-__device__ __forceinline__ void count_full(const DomainArgs& a, bool has, uint32_t rs, uint32_t gs) {
+// grain and warp (full cells of one grain tend to finish together); every lane takes part.  gk: cells taken from
+// the deformed grain by this lane's atomic, gold: its count before (gold == gk: its last cells)
+__device__ __forceinline__ void count_full(const DomainArgs& a, bool has, uint32_t rs, uint32_t gs, uint32_t& gk, uint32_t& gold) {
     const int lane = threadIdx.x & 31;
     const uint32_t act = __ballot_sync(0xFFFFFFFFu, has);
+    if (!act) return;
     const uint32_t mr = __match_any_sync(0xFFFFFFFFu, has ? rs : 0xFFFFFFFFu) & act;
     const uint32_t mg = __match_any_sync(0xFFFFFFFFu, has ? gs : 0xFFFFFFFFu) & act;
     if (has && (__ffs(mr) - 1) == lane) atomicAdd(&a.rxg_cnt[rs], (uint32_t)__popc(mr));
     if (has && (__ffs(mg) - 1) == lane) {
-        const uint32_t k = (uint32_t)__popc(mg);
-        const uint32_t old = atomicSub(&a.defg_cnt[gs], k);
-        if (old == k) {
-            const uint32_t q = atomicAdd(&a.st->ndepleted, 1u);
-            if (q < a.ndefg) a.depleted[q] = gs;
-        }
+        gk = (uint32_t)__popc(mg);
+        gold = atomicSub(&a.defg_cnt[gs], gk);
     }
 }
 
@@ -1809,6 +1887,7 @@ __device__ __forceinline__ void new_cell(const DomainArgs& a, const DFront& dst,
     }
 }
 
+constexpr uint32_t kCommitWins = 1024;  // new cells of a tile listed at a time (a full cell infects about one)
 template <bool FP32, bool ONE>
 __global__ void __launch_bounds__(kBlock, ONE ? 4 : 3) k_commit(int base, int ndom, uint32_t grow_tile) {
     __shared__ uint32_t s_pre[kMaxSegs + 1];
@@ -1925,7 +2004,12 @@ __global__ void __launch_bounds__(kBlock, ONE ? 4 : 3) k_commit(int base, int nd
             if (!FP32) ((double*)src.fill)[slot] = 0.0;
             else { ((float*)src.fill)[slot] = 0.0f; src.comp[slot] = 0.0f; }
         }
-        count_full(a, f < F, rsrc, gsrc);
+        uint32_t gk = 0, gold = 0;
+        count_full(a, f < F, rsrc, gsrc, gk, gold);
+        if (gk && gold == gk) {
+            const uint32_t n = atomicAdd(&a.st->ndepleted, 1u);
+            if (n < a.ndefg) a.depleted[n] = gsrc;
+        }
         __syncthreads();
     }
     if (cur >= 0) flush_new(c_args[base + cur], pmax, ntag);
