@@ -431,7 +431,7 @@ __device__ __forceinline__ void fuse_grow(const DomainArgs& a, const DFront& fr,
                 vel[k] = -1.0f;
                 if (!((act >> k) & 1u)) continue;
                 if (d & kPend) vel[k] = (float)answered_velocity(a, fr, s + k, d, ((const uint32_t*)fr.vel)[s + k]);
-                else vel[k] = (float)velocity_from_mobility(a, mo[k], g[k], d & kCodeMask);
+                else vel[k] = velocity32_from_mobility(a, mo[k], g[k], d & kCodeMask);
             }
             if (whole) X::store(pv, vel);
             else

@@ -38,6 +38,7 @@
 #pragma once
 #include <cstdint>
 #include "device_common.cuh"
+#include "velocity32.h"
 
 namespace score {
 
@@ -204,6 +205,17 @@ __device__ __forceinline__ double velocity_from_force(double m, double p, int co
 }
 __device__ __forceinline__ double velocity_from_mobility(const DomainArgs& a, double m, uint32_t defg, int code) {
     return velocity_from_force(m, a.pforce[defg], code);
+}
+// the same as the FP32 fronts keep it, (float) of the above
+__device__ __forceinline__ float velocity32_from_force(double m, double p, int code) {
+    const long long b = __double_as_longlong(p);
+    if (!(b > __double_as_longlong(5.0e-16) && b <= 0x7FF0000000000000ll)) return -1.0f;
+    float v;
+    if (velocity32((uint64_t)__double_as_longlong(m), (uint64_t)b, (uint32_t)code, v)) return v;
+    return (float)__dmul_rn(__dmul_rn(m, p), shape_factor((uint32_t)code));
+}
+__device__ __forceinline__ float velocity32_from_mobility(const DomainArgs& a, double m, uint32_t defg, int code) {
+    return velocity32_from_force(m, a.pforce[defg], code);
 }
 __device__ __forceinline__ double velocity_factor(const DomainArgs& a, double P, uint32_t defg, int code) {
     return velocity_from_mobility(a, mobility(a, P), defg, code);
@@ -586,7 +598,7 @@ __device__ __forceinline__ uint32_t grow_items(const DomainArgs& a, const DFront
                     const uint32_t slot = base + (uint32_t)(k * 32);
                     if ((act >> k) & 1u) {
                         if (d[k] & kPend) vel[j] = (float)answered_velocity(a, fr, slot, d[k], ((const uint32_t*)fr.vel)[slot]);
-                        else vel[j] = (float)velocity_from_mobility(a, mo[j], g[j], d[k] & kCodeMask);
+                        else vel[j] = velocity32_from_mobility(a, mo[j], g[j], d[k] & kCodeMask);
                         ((float*)fr.vel)[slot] = vel[j];
                     }
                 }
@@ -604,7 +616,7 @@ __device__ __forceinline__ uint32_t grow_items(const DomainArgs& a, const DFront
                             const double P = __longlong_as_double((long long)a.ptab[(unsigned long long)fr.rxg[slot] * a.ndefg + g]);
                             const double mo = mobility(a, P);
                             fr.mob[slot] = mo;
-                            vel[j] = (float)velocity_from_mobility(a, mo, g, d[k] & kCodeMask);
+                            vel[j] = velocity32_from_mobility(a, mo, g, d[k] & kCodeMask);
                         }
                         ((float*)fr.vel)[slot] = vel[j];
                         fill[j] = ((const float*)fr.fill)[slot];
@@ -1867,14 +1879,14 @@ __device__ __forceinline__ void new_cell(const DomainArgs& a, const DFront& dst,
     if (lookup_p(a, rs, gt, P, tag)) {
         const double mo = mobility(a, P);
         dst.mob[ns] = mo;
-        const double v = velocity_from_force(mo, pf, (int)code);
         if (!FP32) {
+            const double v = velocity_from_force(mo, pf, (int)code);
             // the increment with this step's dt: valid next step unless dt changes, when
             // k_grow_fill recomputes every increment from vel anyway
             ((double*)dst.vel)[ns] = v;
             dst.inc[ns] = __double_as_longlong(v) >= 0 ? __dmul_rn(__dmul_rn(v, a.dt), a.cinv) : v;
         } else {
-            ((float*)dst.vel)[ns] = (float)v;
+            ((float*)dst.vel)[ns] = velocity32_from_force(mo, pf, (int)code);
         }
         dst.dir[ns] = (uint8_t)code;
         if (P > pmax) pmax = P;
