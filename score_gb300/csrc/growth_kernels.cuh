@@ -192,8 +192,16 @@ __device__ __forceinline__ bool target_of(const DomainArgs& a, int L, int x, int
 
 // mobility m(P) of the reference (get_currentintrinsicmobility, SCORE_Kernel.cpp:5459-5470)
 __device__ __forceinline__ double mobility(const DomainArgs& a, double P) {
-    if (a.mobility_model == 2) return __dmul_rn(P, a.mRH);
-    if (P < 0.0) return a.mLAGB;
+    // the constants by integers (FP64, compares included, runs at 1/64 rate): 94 % of the pairs.  0 mGS + 1 mHAGB is
+    // mHAGB and 1 mGS + 0 mHAGB is mGS where both are finite and not negative (384^3 sheets 61.4 ms, now 60.6; 64^3
+    // 13.2, now 13.1)
+    const unsigned long long b = (unsigned long long)__double_as_longlong(P);
+    if (a.mobility_model == 2) return b == 0x3FF0000000000000ull ? a.mRH : __dmul_rn(P, a.mRH);
+    if (b > 0x8000000000000000ull && b <= 0xFFF0000000000000ull) return a.mLAGB;  // P < 0
+    if (((uint32_t)__double2hiint(a.mGS) < 0x7FF00000u) & ((uint32_t)__double2hiint(a.mHAGB) < 0x7FF00000u)) {
+        if (b == 0ull) return a.mHAGB;
+        if (b == 0x3FF0000000000000ull) return a.mGS;
+    }
     return __dadd_rn(__dmul_rn(P, a.mGS), __dmul_rn(__dsub_rn(1.0, P), a.mHAGB));
 }
 // velocity factor (m p) f_geo, or -1 when the driving force is not above 5e-16
@@ -1889,7 +1897,8 @@ __device__ __forceinline__ void new_cell(const DomainArgs& a, const DFront& dst,
             ((float*)dst.vel)[ns] = velocity32_from_force(mo, pf, (int)code);
         }
         dst.dir[ns] = (uint8_t)code;
-        if (P > pmax) pmax = P;
+        // P > pmax >= 0 by integers
+        if (__double_as_longlong(P) > __double_as_longlong(pmax) && __double_as_longlong(P) <= 0x7FF0000000000000ll) pmax = P;
     } else {
         // vel holds the answer tag until the next k_grow_fill
         if (!FP32) ((unsigned long long*)dst.vel)[ns] = tag;
