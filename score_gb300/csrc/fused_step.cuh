@@ -3,7 +3,7 @@
 // What bounds such a domain is neither bytes nor operations but the chain of a step: five or six
 // launches, each with its own start, constant-cache misses and dependent loads, then a stream
 // synchronization and the host's master block (64^3 domain, front of 30 k slots: 51 us a step, of which the
-// bytes take 0.1; 128^3: 59 us; here 25 and 28).  A group of blocks steps one domain inside one
+// bytes take 0.1; 128^3: 59 us; here 24 and 28).  A group of blocks steps one domain inside one
 // cooperative launch:
 //   A  fill of the group's tiles, 2 or 4 consecutive slots a thread; full cells into records; the 26 infection
 //      attempts of every full cell, four lanes a cell.  The attempt ordinal is 26 s + d with s the

@@ -15,16 +15,17 @@
 //
 // Every ordered compaction (FullRX list, recycle list, slot ranks of new cells) is a
 // count pass that also adds its counts into supertile sums, and a write pass that
-// takes each tile's exclusive prefix from the supertile and tile counts: no block
-// ever waits on another one.
+// takes each tile's exclusive prefix from the supertile and tile counts: no block of
+// these kernels waits on another one.  (The steps of small fronts run inside one launch whose
+// blocks do, with bounded waits: k_steps_fused.)
 //   k_grow_fill   per list: fill update of every ACTIVE slot in [0, next_never);
 //                 1-bit masks of full and INACTIVE slots, per-warp counts; Sv count.
 //   k_grow_lists  FullRX list and capped recycle list, in slot order.
-//   k_claim   one thread per full cell: the 26 infection attempts in the reference's
+//   k_claim   four lanes per full cell: the 26 infection attempts in the reference's
 //             order; a still-deformed target gets atomicMin(claim, attempt ordinal),
 //             where ordinal = 26 * (full-cell rank, Inside list first) + direction rank.
-//             The thread records which attempts it made (26-bit mask).
-//   k_resolve one thread per full cell: attempts whose claim holds the own ordinal
+//             The attempts made are recorded (26-bit mask).
+//   k_resolve four lanes per full cell: attempts whose claim holds the own ordinal
 //             won; per-tile win counts per destination list.
 //   k_commit  winners are ranked per destination list in full-cell then direction
 //             order and take recycled slots first, then appended slots, like
