@@ -1755,6 +1755,11 @@ namespace {
 // motion for 2,000 steps 235 / 236 / 171 / 171, FP64 512^3 104.3 / 103.7 / 103.6 / 105.9, FP32 384^3 with recovery
 // 160 / 132 / 131 / 131 (211 with none).
 constexpr uint64_t kFuseSlots = 8ull << 20;
+// Slots a block of all the launch's domains: a batch's blocks are shared out to its domains, and beyond this the separate
+// kernels, which put every SM on every domain, gain more than their launches cost.  64 domains in two groups (22 M
+// slots a group on 76 blocks at the end): 284 ms a run without this limit, 249 at 193 K a block, 253 at 221 K, 261 at
+// 248 K; 48 in one group (31 M slots on 152 blocks): 174 without, 185 at 166 K.
+constexpr uint64_t kFuseBlockSlots = 200ull << 10;
 // Slots a block from which a thread takes 4 slots a tile instead of 2: fewer, wider accesses (16-domain batch: fill
 // 42 us a step with 2, 23 with 4), but half the tiles to spread over the blocks.
 constexpr uint64_t kFuseWide = 4096;
@@ -1808,13 +1813,16 @@ struct FuseServe {
 // direct launches (use_graph 0, the autotuner) keep the separate kernels.
 bool Engine::fused_ok() const {
     if (!fuse || !use_graph) return false;
-    uint64_t nrun = 0, tiles = 0;
+    uint64_t nrun = 0, tiles = 0, slots = 0;
     for (const score_ctx* c : dom) {
         if (!c->running) continue;
         ++nrun;
         tiles += fuse_tiles(c, 4);
-        if ((uint64_t)c->next_never[0] + c->next_never[1] > kFuseSlots) return false;
+        const uint64_t s = (uint64_t)c->next_never[0] + c->next_never[1];
+        if (s > kFuseSlots) return false;
+        slots += s;
     }
+    if (slots > kFuseBlockSlots * (uint64_t)fuse_sms) return false;
     // a domain's blocks follow its share of the tiles: kFuseMaxLocal tiles a block with room to grow
     return nrun > 0 && nrun < (uint64_t)fuse_sms && tiles + 4 * nrun <= (kFuseMaxLocal / 2) * ((uint64_t)fuse_sms - nrun);
 }

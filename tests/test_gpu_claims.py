@@ -27,3 +27,23 @@ def test_batch_by_separate_kernels(gpu, tmp_path, names):
         assert b.timing().kernel_launches >= 5 * steps
         for i, n in enumerate(names):
             assert_same(b.trace(i), b.labels(i), *b.grain_counts(i), refs[n])
+
+
+def test_batch_changes_paths_on_the_way(gpu, tmp_path):
+    """A batch whose fronts outgrow the launch's blocks goes on with the separate kernels, and back."""
+    names = ["odd_periodic", "one_nucleus", "many_full", "thin"]
+    cases = [make(n, tmp_path) for n in names]
+    with sg.Batch([p for p, _ in cases]) as b:
+        for i, (_, d) in enumerate(cases):
+            b.load_domain(i, d)
+        b.place_nuclei()
+        traces = [[] for _ in names]
+        for k in range(6):
+            b.set_tune(use_graph=k % 2)
+            b.run_until(max_steps=5)
+            for i in range(len(names)):
+                traces[i] += b.trace(i)
+        b.set_tune(use_graph=1)
+        b.run_until()
+        for i, (p, d) in enumerate(cases):
+            assert_same(traces[i] + b.trace(i), b.labels(i), *b.grain_counts(i), oracle.run(p, d))
