@@ -40,8 +40,8 @@ constexpr uint32_t kFuseMaxLocal = 512;                   // tiles of one block
 constexpr uint32_t kFuseRec = 2048;                       // full cells of a block and step kept in shared memory
 constexpr uint32_t kFuseMask = 2048;                      // mask words of a block kept in shared memory
 constexpr uint32_t kFuseWins = 4096;                      // new cells listed at a time
-constexpr uint32_t kFuseSpin = 1u << 22;                  // polls of a group wait before it gives up (seconds)
-constexpr uint32_t kFuseHostSpin = 1u << 12;              // polls of the host's answer before the group leaves (milliseconds)
+constexpr uint32_t kFuseSpin = 1u << 22;                  // polls of a group wait before it gives up (seconds), at most
+constexpr uint32_t kFuseHostSpin = 1u << 12;              // polls of the host's answer before the group leaves (milliseconds), at most
 
 // the host's word: step number (equality is all that counts) and flags
 constexpr uint32_t kCmdLeave = 1u;        // no further step in this launch
@@ -68,6 +68,7 @@ struct FuseDom {
 struct FuseMap {
     uint16_t first[kMaxDomains + 1];   // blocks [first[i], first[i + 1]) step domain i
     uint32_t ndom;
+    uint32_t group_polls, host_polls;  // limits of the waits
     uint32_t seq[kMaxDomains];         // step number of domain i's first command in this launch
 };
 
@@ -119,14 +120,14 @@ struct FuseShared {
 
 // Arrival of the block at its group's barrier and, with `wait`, the wait for the whole group.  target: arrivals
 // of the launch so far when everyone is there.  False (for the whole block) when the wait gave up.
-__device__ __forceinline__ bool group_barrier(FuseShared& sh, uint32_t* bar, uint32_t G, uint32_t target, bool wait) {
+__device__ __forceinline__ bool group_barrier(FuseShared& sh, uint32_t* bar, uint32_t G, uint32_t target, uint32_t polls, bool wait) {
     __syncthreads();
     if (G == 1) return true;
     if (threadIdx.x == 0) {
         fence_gpu();   // cumulative: the block's stores, ordered before thread 0 by the block barrier
         asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         bool ok = !wait;
-        for (uint32_t k = 0; !ok && k < kFuseSpin; ++k) ok = (int32_t)(ld_relaxed_gpu(bar) - target) >= 0;
+        for (uint32_t k = 0; !ok && k < polls; ++k) ok = (int32_t)(ld_relaxed_gpu(bar) - target) >= 0;
         fence_gpu();
         sh.ok = ok ? 1u : 0u;
     }
@@ -514,7 +515,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             if (threadIdx.x == 0) {
                 uint32_t w = 0;
                 bool ok = false;
-                for (uint32_t k = 0; !ok && k < kFuseHostSpin; ++k) {
+                for (uint32_t k = 0; !ok && k < map.host_polls; ++k) {
                     w = ld_relaxed_sys(&fh->cmd);
                     ok = (w >> kCmdShift) == seq;
                 }
@@ -539,7 +540,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             if (threadIdx.x == 0) {
                 uint32_t w = 0;
                 bool ok = false;
-                for (uint32_t k = 0; !ok && k < kFuseSpin; ++k) {
+                for (uint32_t k = 0; !ok && k < map.group_polls; ++k) {
                     w = ld_relaxed_gpu(&fd->go);
                     ok = (w >> kCmdShift) == seq;
                 }
@@ -568,7 +569,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             const double* src = fd->pay.pf_src;
             for (uint32_t g = rank * kFuse + threadIdx.x; g < a.ndefg; g += G * kFuse) ((double*)a.pforce)[g] = src[g];
             arrived += G;
-            if (!group_barrier(sh, &fd->bar, G, arrived, true)) { if (threadIdx.x == 0) fuse_gave_up(st, 1u, rank, arrived); return; }
+            if (!group_barrier(sh, &fd->bar, G, arrived, map.group_polls, true)) { if (threadIdx.x == 0) fuse_gave_up(st, 1u, rank, arrived); return; }
         }
         __syncthreads();
 
@@ -676,7 +677,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             }
         }
         arrived += G;
-        if (!group_barrier(sh, &fd->bar, G, arrived, true)) { if (threadIdx.x == 0) fuse_gave_up(st, 2u, rank, arrived); return; }
+        if (!group_barrier(sh, &fd->bar, G, arrived, map.group_polls, true)) { if (threadIdx.x == 0) fuse_gave_up(st, 2u, rank, arrived); return; }
         const uint32_t t_a = now_ns();
 
         // ---- B: recycle list, wins
@@ -741,7 +742,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
         __syncthreads();
         for (uint32_t lt = threadIdx.x; lt < nlt; lt += kFuse) cntB[rank + lt * G] = make_uint2(sh.tw[0][lt], sh.tw[1][lt]);
         arrived += G;
-        if (!group_barrier(sh, &fd->bar, G, arrived, true)) { if (threadIdx.x == 0) fuse_gave_up(st, 3u, rank, arrived); return; }
+        if (!group_barrier(sh, &fd->bar, G, arrived, map.group_polls, true)) { if (threadIdx.x == 0) fuse_gave_up(st, 3u, rank, arrived); return; }
         const uint32_t t_b = now_ns();
 
         // ---- C: commit
@@ -822,7 +823,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
         }
         if (__any_sync(0xFFFFFFFFu, pmax > 0.0 || ntag)) flush_new(a, pmax, ntag);
         arrived += G;
-        if (!group_barrier(sh, &fd->bar, G, arrived, first)) { if (threadIdx.x == 0) fuse_gave_up(st, 4u, rank, arrived); return; }
+        if (!group_barrier(sh, &fd->bar, G, arrived, map.group_polls, first)) { if (threadIdx.x == 0) fuse_gave_up(st, 4u, rank, arrived); return; }
         // the lists' ends after this step, the same in every block
         const uint32_t p0 = n0, p1 = n1;
         if (W0 > nrec0) n0 += W0 - nrec0;

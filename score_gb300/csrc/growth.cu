@@ -682,6 +682,29 @@ private:
     uint64_t round_ = 0;  // only the calling thread starts rounds
 };
 
+// Slots of a domain's front up to which its steps run inside one launch.  A fused step saves the separate
+// kernels' fixed cost (about 50 us) but streams a large front with half their loads in flight.  Measured per run,
+// limits of 2 / 4 / 8 / 14 M slots: FP64 384^3 rolled sheet 67.9 / 68.1 / 63.5 / 63.6 ms, the same with few cells in
+// motion for 2,000 steps 235 / 236 / 171 / 171, FP64 512^3 104.3 / 103.7 / 103.6 / 105.9, FP32 384^3 with recovery
+// 160 / 132 / 131 / 131 (211 with none).
+constexpr uint64_t kFuseSlots = 8ull << 20;
+// Slots a block of all the launch's domains: a batch's blocks are shared out to its domains, and beyond this the separate
+// kernels, which put every SM on every domain, gain more than their launches cost.  64 domains in two groups (22 M
+// slots a group on 76 blocks at the end): 284 ms a run without this limit, 249 at 193 K a block, 253 at 221 K, 261 at
+// 248 K; 48 in one group (31 M slots on 152 blocks): 174 without, 185 at 166 K.
+constexpr uint64_t kFuseBlockSlots = 200ull << 10;
+// Slots a block from which a thread takes 4 slots a tile instead of 2: fewer, wider accesses (16-domain batch: fill
+// 42 us a step with 2, 23 with 4), but half the tiles to spread over the blocks.
+constexpr uint64_t kFuseWide = 4096;
+
+// The limits of an engine's fused steps.  Results do not depend on them: tests lower them, so that small domains take
+// every path (score_internal_step_limits), never raise them.
+struct StepLimits {
+    uint32_t host_polls = kFuseHostSpin, group_polls = kFuseSpin;
+    uint32_t wide = (uint32_t)kFuseWide, block_slots = (uint32_t)kFuseBlockSlots;
+    uint64_t slots = kFuseSlots;
+};
+
 struct Engine {
     int device = 0, sms = 1;
     cudaStream_t stream = nullptr;
@@ -783,6 +806,7 @@ struct Engine {
     void get_tune(score_tune* out) const;
     int set_tune(const score_tune* t);
     void mark_run_start() { cudaEventRecord(ev[5], stream); run_steps = 0; }
+    StepLimits lim;
     bool fuse = false;                 // cooperative launches of k_steps_fused are possible
     int fuse_sms = 1;                  // blocks of one of them (batches share the SMs between their engines)
     bool sample_step() const { return cfg.timing_every > 0 && run_steps % (uint64_t)cfg.timing_every == 0; }
@@ -1749,21 +1773,6 @@ int Engine::mark_run_end() {
 // ------------------------------------------------------------------ many steps in one launch
 namespace {
 
-// Slots of a domain's front up to which its steps run inside one launch.  A fused step saves the separate
-// kernels' fixed cost (about 50 us) but streams a large front with half their loads in flight.  Measured per run,
-// limits of 2 / 4 / 8 / 14 M slots: FP64 384^3 rolled sheet 67.9 / 68.1 / 63.5 / 63.6 ms, the same with few cells in
-// motion for 2,000 steps 235 / 236 / 171 / 171, FP64 512^3 104.3 / 103.7 / 103.6 / 105.9, FP32 384^3 with recovery
-// 160 / 132 / 131 / 131 (211 with none).
-constexpr uint64_t kFuseSlots = 8ull << 20;
-// Slots a block of all the launch's domains: a batch's blocks are shared out to its domains, and beyond this the separate
-// kernels, which put every SM on every domain, gain more than their launches cost.  64 domains in two groups (22 M
-// slots a group on 76 blocks at the end): 284 ms a run without this limit, 249 at 193 K a block, 253 at 221 K, 261 at
-// 248 K; 48 in one group (31 M slots on 152 blocks): 174 without, 185 at 166 K.
-constexpr uint64_t kFuseBlockSlots = 200ull << 10;
-// Slots a block from which a thread takes 4 slots a tile instead of 2: fewer, wider accesses (16-domain batch: fill
-// 42 us a step with 2, 23 with 4), but half the tiles to spread over the blocks.
-constexpr uint64_t kFuseWide = 4096;
-
 uint32_t fuse_tiles(const score_ctx* c, int items) {
     const uint32_t tile = (uint32_t)(kFuse * items);
     return (c->next_never[0] + tile - 1) / tile + (c->next_never[1] + tile - 1) / tile;
@@ -1819,10 +1828,10 @@ bool Engine::fused_ok() const {
         ++nrun;
         tiles += fuse_tiles(c, 4);
         const uint64_t s = (uint64_t)c->next_never[0] + c->next_never[1];
-        if (s > kFuseSlots) return false;
+        if (s > lim.slots) return false;
         slots += s;
     }
-    if (slots > kFuseBlockSlots * (uint64_t)fuse_sms) return false;
+    if (slots > (uint64_t)lim.block_slots * (uint64_t)fuse_sms) return false;
     // a domain's blocks follow its share of the tiles: kFuseMaxLocal tiles a block with room to grow
     return nrun > 0 && nrun < (uint64_t)fuse_sms && tiles + 4 * nrun <= (kFuseMaxLocal / 2) * ((uint64_t)fuse_sms - nrun);
 }
@@ -1838,7 +1847,7 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
     for (const score_ctx* c : dom)
         if (c->running) slots += (uint64_t)c->next_never[0] + c->next_never[1];
     // 4 slots a thread and tile once every block has several tiles of 2
-    const int items = slots >= kFuseWide * (uint64_t)fuse_sms ? 4 : 2;
+    const int items = slots >= (uint64_t)lim.wide * (uint64_t)fuse_sms ? 4 : 2;
     std::vector<FuseServe> sv;
     FuseMap map{};
     uint64_t work = 0;
@@ -1873,6 +1882,8 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
         }
         map.first[n] = (uint16_t)total;
         map.ndom = (uint32_t)n;
+        map.group_polls = lim.group_polls;
+        map.host_polls = lim.host_polls;
     }
     cudaError_t e = cudaSuccess;
     if (args_dirty || memcmp(h_args, h_args_dev.data(), (size_t)n * sizeof(DomainArgs)) != 0) {
@@ -1978,7 +1989,7 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
         f.status = finish_step(f);
         const double xt = x_target < 0 ? c->prm.xmax : x_target;
         const bool needs = f.status == SCORE_OK && (c->log_info.size() != logged || fuse_needs_stream(c) ||
-                           (uint64_t)c->next_never[0] + c->next_never[1] > kFuseSlots || fuse_tiles(c, items) > std::min(kFuseMaxLocal * f.blocks, kFuseMaxTiles - 512));
+                           (uint64_t)c->next_never[0] + c->next_never[1] > lim.slots || fuse_tiles(c, items) > std::min(kFuseMaxLocal * f.blocks, kFuseMaxTiles - 512));
         if (f.status != SCORE_OK || needs) stop.store(true, std::memory_order_relaxed);
         if (f.status != SCORE_OK || needs || one || domain_done(c, xt) || (max_steps && done[f.i] >= max_steps) ||
             stop.load(std::memory_order_relaxed)) {
@@ -2945,6 +2956,28 @@ int score_batch_autotune(score_batch* b, double x_target, uint32_t max_steps, sc
 }
 
 }  // extern "C"
+
+// Lower limits of a context's or a batch's fused steps, for the tests; not part of the C interface (the header does not
+// declare it).  null: the defaults.
+namespace {
+StepLimits lowered(const StepLimits* l) {
+    const StepLimits d;
+    if (!l) return d;
+    StepLimits r;
+    r.host_polls = std::max(1u, std::min(l->host_polls, d.host_polls));
+    r.group_polls = std::max(1u, std::min(l->group_polls, d.group_polls));
+    r.wide = std::min(l->wide, d.wide);
+    r.block_slots = std::min(l->block_slots, d.block_slots);
+    r.slots = std::min(l->slots, d.slots);
+    return r;
+}
+}  // namespace
+
+extern "C" int score_internal_step_limits(score_ctx* c, score_batch* b, const StepLimits* l) {
+    if (c) c->eng->lim = lowered(l);
+    if (b) for (auto& E : b->engs) E->lim = lowered(l);
+    return c || b ? SCORE_OK : SCORE_ERR_ARG;
+}
 
 // ------------------------------------------------------------------ no-allocation table
 // Device FP64 mobility-weight table P(rxg, defg) for all pairs, with the grid-wide

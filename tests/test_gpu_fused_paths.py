@@ -1,0 +1,102 @@
+"""Paths of the fused steps that small domains reach only with lower limits: four slots a thread, fronts that outgrow the
+launch and its blocks on the way, and groups that leave before the host's answer (the next launch, or the separate
+kernels, take the command again).  FP64: the oracle's bits; FP32: the separate kernels' bits.
+"""
+import numpy as np
+import pytest
+
+import oracle
+import score_gb300 as sg
+from _limits import set_limits
+from test_gpu_fused import CASES, make
+from test_gpu_parity import assert_same
+
+pytestmark = pytest.mark.gpu
+
+
+def run(p, d, use_graph=1, **lim):
+    """trace, labels, counts and launches of a run"""
+    with sg.GrowthMachine(p) as gm:
+        set_limits(gm, **lim)
+        gm.set_tune(use_graph=use_graph)
+        gm.load_domain(d)
+        gm.place_nuclei()
+        n0 = gm.timing().kernel_launches
+        tr = gm.run_until()
+        n = gm.timing().kernel_launches - n0
+        return tr, gm.labels(), gm.grain_counts(), n
+
+
+def as_array(tr):
+    return np.array([(s.t, s.Xcells, s.Sv, s.Pmax, s.n_new) for s in tr])
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_four_slots_a_thread(gpu, tmp_path, name):
+    p, d = make(name, tmp_path)
+    tr, labels, counts, n = run(p, d, wide=0)
+    assert n < 5 * len(tr), "the separate kernels ran"
+    assert_same(tr, labels, *counts, oracle.run(p, d))
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_four_slots_a_thread_fp32(gpu, tmp_path, name):
+    p, d = make(name, tmp_path, precision=1)
+    tr, labels, counts, n = run(p, d, wide=0)
+    assert n < 5 * len(tr), "the separate kernels ran"
+    ref = run(p, d, use_graph=0)
+    assert np.array_equal(as_array(tr), as_array(ref[0])) and np.array_equal(labels, ref[1])
+    assert all(np.array_equal(a, b) for a, b in zip(counts, ref[2]))
+
+
+@pytest.mark.parametrize("name", ["odd_periodic", "heating", "recovery_nuclei", "defrag"])
+def test_front_outgrows_the_launch(gpu, tmp_path, name):
+    """Fused below 3,000 slots, separate kernels above."""
+    p, d = make(name, tmp_path)
+    ref = oracle.run(p, d)
+    tr, labels, counts, n = run(p, d, slots=3000)
+    small = sum(sum(s.next_never) <= 3000 for s in tr)
+    assert 0 < small < len(tr) - 5 and n > 5 * (len(tr) - small - 1)
+    assert_same(tr, labels, *counts, ref)
+
+
+def test_batch_outgrows_its_blocks(gpu, tmp_path):
+    """16 slots a block of the launch: the batch goes on with the separate kernels."""
+    names = ["odd_periodic", "one_nucleus", "heating", "recovery_nuclei"]
+    cases = [make(n, tmp_path) for n in names]
+    with sg.Batch([p for p, _ in cases]) as b:
+        set_limits(b, block_slots=16)
+        for i, (_, d) in enumerate(cases):
+            b.load_domain(i, d)
+        b.place_nuclei()
+        steps = b.run_until()
+        assert steps < b.timing().kernel_launches < 6 * steps, "one path only"
+        for i, (p, d) in enumerate(cases):
+            assert_same(b.trace(i), b.labels(i), *b.grain_counts(i), oracle.run(p, d))
+
+
+# one poll is shorter than a round trip over the host link: nearly every group leaves, with the next command unread
+@pytest.mark.parametrize("lim", [{}, {"slots": 3000}, {"wide": 0}], ids=["next_launch", "separate_kernels", "four_slots"])
+@pytest.mark.parametrize("name", ["odd_periodic", "heating", "heating_rh", "recovery_nuclei", "recovery_mp", "defrag"])
+def test_group_leaves_before_the_answer(gpu, tmp_path, name, lim):
+    p, d = make(name, tmp_path)
+    tr, labels, counts, n = run(p, d, host_polls=1, **lim)
+    fused = sum(sum(s.next_never) <= lim.get("slots", 2**32) for s in tr)
+    assert n >= fused // 2, "the groups stayed"
+    assert_same(tr, labels, *counts, oracle.run(p, d))
+
+
+def test_batch_leaves_before_the_answer(gpu, tmp_path):
+    names = ["odd_periodic", "one_nucleus", "heating", "recovery_nuclei", "defrag", "many_full"]
+    cases = [make(n, tmp_path) for n in names]
+    for kw in ({"host_polls": 1}, {"host_polls": 1, "block_slots": 40}):
+        with sg.Batch([p for p, _ in cases]) as b:
+            set_limits(b, **kw)
+            for i, (_, d) in enumerate(cases):
+                b.load_domain(i, d)
+            b.place_nuclei()
+            b.run_until(max_steps=7)
+            first = [b.trace(i) for i in range(len(names))]
+            b.run_until()
+            for i, (p, d) in enumerate(cases):
+                assert_same(first[i] + b.trace(i), b.labels(i), *b.grain_counts(i), oracle.run(p, d))
