@@ -55,6 +55,9 @@ constexpr uint32_t kCmdForce = 128u;      // new driving forces in payload.pf_sr
 constexpr uint32_t kCmdReplay = 1u << 31; // host only, in place of the step number: a command to give again
 constexpr uint32_t kCmdShift = 8u;
 constexpr uint32_t kCmdSeqMask = 0xFFFFFFu;
+// Step numbers run from 1 to kCmdSeqMask and start again: 0, which `post`, `left` and `go` hold when nothing was written, is
+// none.
+__host__ __device__ __forceinline__ uint32_t fuse_next(uint32_t seq) { return seq == kCmdSeqMask ? 1u : seq + 1u; }
 
 // device memory: one per domain
 struct FuseDom {
@@ -506,7 +509,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
     FuseHost* const fh = &a.box->fuse;
     const bool first = rank == 0;
     uint32_t n0 = st->next_never[0], n1 = st->next_never[1];
-    uint32_t seq = map.seq[dom] & kCmdSeqMask, arrived = 0;
+    uint32_t seq = map.seq[dom], arrived = 0;
     if (threadIdx.x < 26)
         sh.dir[threadIdx.x] = c_dir.v[threadIdx.x];
     for (;;) {
@@ -871,7 +874,7 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             }
         }
         if (w & kCmdLast) return;
-        seq = (seq + 1u) & kCmdSeqMask;
+        seq = fuse_next(seq);
     }
 }
 

@@ -703,6 +703,7 @@ struct StepLimits {
     uint32_t host_polls = kFuseHostSpin, group_polls = kFuseSpin;
     uint32_t wide = (uint32_t)kFuseWide, block_slots = (uint32_t)kFuseBlockSlots;
     uint64_t slots = kFuseSlots;
+    uint32_t number = 0;               // of the next command (1 to kCmdSeqMask; 0: as it is)
 };
 
 struct Engine {
@@ -1902,6 +1903,9 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
         }
         c->fuse_replay = 0;
         f.word |= (c->fuse_seq << kCmdShift) | (one ? kCmdLast : 0u);
+        // numbers come back after 2^24 steps: the device's words of an earlier launch would be taken for this one's
+        c->h_box->fuse.post = 0;
+        c->h_box->fuse.left = 0;
         fuse_store(&c->h_box->fuse.cmd, f.word);
         c->fuse_live = true;
         f.open = true;
@@ -1934,7 +1938,7 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
         f.open = false;
         if (one) return;  // it has left
         fuse_store(&c->h_box->fuse.cmd, (c->fuse_seq << kCmdShift) | kCmdLeave);
-        c->fuse_seq = (c->fuse_seq + 1) & kCmdSeqMask;
+        c->fuse_seq = fuse_next(c->fuse_seq);
     };
     // after the post of a step: the host's part of it, and the next command
     auto finish_step = [&](FuseServe& f) -> int {
@@ -1973,11 +1977,11 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
         if (fuse_load(&h.post) != seq) {
             if (fuse_load(&h.left) != seq) return false;
             f.open = false;  // the group left before it saw the command: the next launch takes the step
-            c->fuse_seq = (seq + 1) & kCmdSeqMask;
+            c->fuse_seq = fuse_next(seq);
             c->fuse_replay = (f.word & ((1u << kCmdShift) - 1u) & ~kCmdLast) | kCmdReplay;
             return true;
         }
-        c->fuse_seq = (seq + 1) & kCmdSeqMask;
+        c->fuse_seq = fuse_next(seq);
         const DevState& hs = c->h_box->snap;
         if (hs.err || hs.nmiss > kBoxMiss || hs.ndepleted > kBoxDep) {
             f.deferred = true;
@@ -2974,8 +2978,13 @@ StepLimits lowered(const StepLimits* l) {
 }  // namespace
 
 extern "C" int score_internal_step_limits(score_ctx* c, score_batch* b, const StepLimits* l) {
-    if (c) c->eng->lim = lowered(l);
-    if (b) for (auto& E : b->engs) E->lim = lowered(l);
+    auto set = [l](Engine& E) {
+        E.lim = lowered(l);
+        if (l && l->number)
+            for (score_ctx* d : E.dom) d->fuse_seq = std::min(l->number, kCmdSeqMask);
+    };
+    if (c) set(*c->eng);
+    if (b) for (auto& E : b->engs) set(*E);
     return c || b ? SCORE_OK : SCORE_ERR_ARG;
 }
 

@@ -100,3 +100,44 @@ def test_batch_leaves_before_the_answer(gpu, tmp_path):
             b.run_until()
             for i, (p, d) in enumerate(cases):
                 assert_same(first[i] + b.trace(i), b.labels(i), *b.grain_counts(i), oracle.run(p, d))
+
+
+@pytest.mark.parametrize("polls", [1, 4096])
+def test_step_numbers_come_back(gpu, tmp_path, polls):
+    """Numbers end at 2^24 - 1: the count passes its end in a run, in single calls, with groups that leave and without, and
+    meets a number again after which a group once left."""
+    last = 2**24 - 1
+    p, d = make("recovery_nuclei", tmp_path)
+    ref = oracle.run(p, d)
+    assert len(ref["trace"]) > 60
+    with sg.GrowthMachine(p) as gm:
+        gm.load_domain(d)
+        for first in (last - 40, last - 1, last, 1):
+            set_limits(gm, number=first, host_polls=polls)
+            gm.place_nuclei()
+            tr = [gm.step() for _ in range(20)]
+            set_limits(gm, host_polls=polls)
+            tr += gm.run_until()
+            assert_same(tr, gm.labels(), *gm.grain_counts(), ref)
+            gm.restart()
+        # every number of a run in which the groups left
+        set_limits(gm, number=1000, host_polls=1)
+        gm.place_nuclei()
+        gm.run_until()
+        gm.restart()
+        set_limits(gm, number=1000)
+        gm.place_nuclei()
+        assert_same(gm.run_until(), gm.labels(), *gm.grain_counts(), ref)
+
+
+def test_step_numbers_come_back_in_a_batch(gpu, tmp_path):
+    names = ["odd_periodic", "heating", "many_full"]
+    cases = [make(n, tmp_path) for n in names]
+    with sg.Batch([p for p, _ in cases]) as b:
+        set_limits(b, number=2**24 - 30)
+        for i, (_, d) in enumerate(cases):
+            b.load_domain(i, d)
+        b.place_nuclei()
+        b.run_until()
+        for i, (p, d) in enumerate(cases):
+            assert_same(b.trace(i), b.labels(i), *b.grain_counts(i), oracle.run(p, d))
