@@ -1177,6 +1177,8 @@ int reset_state(score_ctx* c) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(a.defg_cnt, c->d_defg_cnt_init, (size_t)c->ndefg * 4, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(a.rxg_cnt, 0, std::max<size_t>(c->nrxg, 1) * 4, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_state, 0, sizeof(DevState), st);
+    // a group whose wait gave up leaves its arrivals and its last word: the next launch's barriers would open early
+    if (e == cudaSuccess) e = cudaMemsetAsync(a.fuse, 0, sizeof(FuseDom), st);
     for (int L = 0; L < 2 && e == cudaSuccess; ++L) e = cudaMemsetAsync(a.f[L].scnt, 0, c->scnt_words[L] * 4, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(a.csct, 0, c->csct_words * 4, st);
     if (e != cudaSuccess) return c->cuda_fail(e, "reset domain");
@@ -1188,6 +1190,8 @@ int reset_state(score_ctx* c) {
     for (size_t k = 0; k < c->log_cells.size(); ++k) c->log_cells[k] = c->prm.logpoint_x[k] * (double)c->N;  // log_initialization, :60-62
     memset(&c->h_box->snap, 0, sizeof(DevState));
     c->running = false;
+    c->fuse_live = false;
+    c->fuse_seq = fuse_next(c->fuse_seq);
     c->pre_done = false;
     c->fuse_replay = 0;
     c->pf_pending = false;
@@ -2523,7 +2527,6 @@ int score_load_domain(score_ctx* c, const uint32_t* grid, const double* defg_qua
         if (e == cudaSuccess) e = dalloc((float4**)&a.dfq, ndefg);
         if (e == cudaSuccess) e = dalloc(&c->d_state, 1);
         if (e == cudaSuccess) e = dalloc(&a.fuse, 1);
-        if (e == cudaSuccess) e = cudaMemsetAsync(a.fuse, 0, sizeof(FuseDom), c->stream);
         if (e == cudaSuccess) e = dalloc(&c->d_pforce, ndefg);
         if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_pforce, std::max<size_t>(ndefg, 1) * 16);
         if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_due, kDueMax * sizeof(NucDue));

@@ -7,6 +7,7 @@ import pytest
 
 import oracle
 import score_gb300 as sg
+from score_gb300 import _abi
 from _limits import set_limits
 from test_gpu_fused import CASES, make
 from test_gpu_parity import assert_same
@@ -141,3 +142,27 @@ def test_step_numbers_come_back_in_a_batch(gpu, tmp_path):
         b.run_until()
         for i, (p, d) in enumerate(cases):
             assert_same(b.trace(i), b.labels(i), *b.grain_counts(i), oracle.run(p, d))
+
+
+@pytest.mark.parametrize("again", ["restart", "load"])
+@pytest.mark.parametrize("name", ["odd_periodic", "recovery_nuclei"])
+def test_restart_after_a_wait_gave_up(gpu, tmp_path, name, again):
+    """One poll a wait: the group's first barrier gives up and the run ends with an error; a restart or a load puts the group's
+    words back, and the next run is the oracle's."""
+    p, d = make(name, tmp_path)
+    ref = oracle.run(p, d)
+    with sg.GrowthMachine(p) as gm:
+        gm.load_domain(d)
+        for _ in range(3):
+            gm.place_nuclei()
+            set_limits(gm, group_polls=1)
+            with pytest.raises(sg.ScoreError) as e:
+                gm.run_until()
+            assert e.value.status == _abi.ERR_TIMEOUT
+            with pytest.raises(sg.ScoreError):
+                gm.run_until()
+            set_limits(gm)
+            gm.restart() if again == "restart" else gm.load_domain(d)
+            gm.place_nuclei()
+            assert_same(gm.run_until(), gm.labels(), *gm.grain_counts(), ref)
+            gm.restart()
