@@ -704,6 +704,7 @@ struct StepLimits {
     uint32_t wide = (uint32_t)kFuseWide, block_slots = (uint32_t)kFuseBlockSlots;
     uint64_t slots = kFuseSlots;
     uint32_t number = 0;               // of the next command (1 to kCmdSeqMask; 0: as it is)
+    uint32_t refuse_after = ~0u;       // cooperative launches until one is answered as refused (~0: never)
 };
 
 struct Engine {
@@ -1905,7 +1906,6 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
             f.word = fuse_flags(c);
             c->fuse_sent = fuse_pay(c);
         }
-        c->fuse_replay = 0;
         f.word |= (c->fuse_seq << kCmdShift) | (one ? kCmdLast : 0u);
         // numbers come back after 2^24 steps: the device's words of an earlier launch would be taken for this one's
         c->h_box->fuse.post = 0;
@@ -1918,19 +1918,22 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
         void* args[] = {(void*)&map, (void*)&base};
         const void* k = items == 4 ? (fp32 ? (const void*)k_steps_fused<true, 4> : (const void*)k_steps_fused<false, 4>)
                                    : (fp32 ? (const void*)k_steps_fused<true, 2> : (const void*)k_steps_fused<false, 2>);
-        e = cudaLaunchCooperativeKernel(k, dim3(total), dim3(kFuse), args, sizeof(FuseShared), stream);
+        if (lim.refuse_after == 0) e = cudaErrorCooperativeLaunchTooLarge;
+        else e = cudaLaunchCooperativeKernel(k, dim3(total), dim3(kFuse), args, sizeof(FuseShared), stream);
+        if (lim.refuse_after != ~0u) --lim.refuse_after;
     }
     if (e != cudaSuccess) {
         for (FuseServe& f : sv) f.c->fuse_live = false;
         if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources) {
             cudaGetLastError();
-            fuse = false;  // the separate kernels from now on
+            fuse = false;  // the separate kernels from now on; they take a command to give again too
             return SCORE_OK;
         }
         for (score_ctx* c : dom) c->failed = true;
         return fail(SCORE_ERR_CUDA, std::string("growth steps: ") + cudaGetErrorString(e));
     }
     launches += 1;
+    for (FuseServe& f : sv) f.c->fuse_replay = 0;
     std::atomic<bool> stop{false};
     const double bpu = fp32 ? 21.0 : 25.0;
     const uint64_t sample0 = run_steps;
@@ -2595,7 +2598,15 @@ int score_step(score_ctx* c, score_step_stats* out) {
     if (c->failed) return SCORE_ERR_STATE;  // a device error left the front lists undefined
     c->running = true;
     std::vector<uint32_t> done(1, 0);
-    const int s = c->eng->fused_ok() ? c->eng->fused_session(2.0, 1, true, done) : c->eng->step(c->eng->sample_step());
+    int s = SCORE_OK;
+    while (s == SCORE_OK && done[0] == 0) {  // a launch that is refused, or that its group leaves early, makes no step
+        if (c->eng->fused_ok()) {
+            s = c->eng->fused_session(2.0, 1, true, done);
+        } else {
+            s = c->eng->step(c->eng->sample_step());
+            done[0] = 1;
+        }
+    }
     c->running = false;
     if (s != SCORE_OK) { if (c->err.empty()) c->err = c->eng->err; return s; }
     if (out) *out = c->last;
@@ -2976,6 +2987,7 @@ StepLimits lowered(const StepLimits* l) {
     r.wide = std::min(l->wide, d.wide);
     r.block_slots = std::min(l->block_slots, d.block_slots);
     r.slots = std::min(l->slots, d.slots);
+    r.refuse_after = l->refuse_after;
     return r;
 }
 }  // namespace

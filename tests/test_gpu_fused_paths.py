@@ -166,3 +166,21 @@ def test_restart_after_a_wait_gave_up(gpu, tmp_path, name, again):
             gm.place_nuclei()
             assert_same(gm.run_until(), gm.labels(), *gm.grain_counts(), ref)
             gm.restart()
+
+
+@pytest.mark.parametrize("at", [0, 1, 30])
+@pytest.mark.parametrize("name", ["odd_periodic", "recovery_nuclei"])
+def test_refused_launch(gpu, tmp_path, name, at):
+    """A cooperative launch that is refused (the answer comes from a stand-in for the call): the separate kernels make the
+    step, one call as well as a run, also the step of a command that its group did not read."""
+    p, d = make(name, tmp_path)
+    ref = oracle.run(p, d)
+    n = len(ref["trace"])
+    for singles, polls in ((n, 4096), (0, 4096), (0, 1)):
+        with sg.GrowthMachine(p) as gm:
+            set_limits(gm, refuse_after=at, host_polls=polls)
+            gm.load_domain(d)
+            gm.place_nuclei()
+            tr = [gm.step() for _ in range(singles)]
+            tr += gm.run_until()
+            assert_same(tr, gm.labels(), *gm.grain_counts(), ref)
