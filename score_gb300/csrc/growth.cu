@@ -2114,7 +2114,8 @@ int Engine::run_until(double x_target, uint32_t max_steps, uint32_t* steps_done)
         for (size_t i = 0; i < dom.size(); ++i) {
             score_ctx* c = dom[i];
             const double xt = x_target < 0 ? c->prm.xmax : x_target;
-            c->running = c->loaded && !c->failed && !domain_done(c, xt) && !(max_steps && done[i] >= max_steps);
+            // a step that is prepared and waits for its next launch belongs to the run: its time has moved on already
+            c->running = c->loaded && !c->failed && (c->pre_done || (!domain_done(c, xt) && !(max_steps && done[i] >= max_steps)));
             nrun += c->running;
         }
         if (nrun == 0) break;

@@ -184,3 +184,17 @@ def test_refused_launch(gpu, tmp_path, name, at):
             tr = [gm.step() for _ in range(singles)]
             tr += gm.run_until()
             assert_same(tr, gm.labels(), *gm.grain_counts(), ref)
+
+
+def test_stop_rules_wait_for_the_pending_step(gpu, tmp_path):
+    """A run that ends by time: the time moves on while a step runs, also when its group has left before it; the step still
+    belongs to the run."""
+    p, d = make("recovery_nuclei", tmp_path)
+    t = oracle.run(p, d)["trace"]["t"]
+    for k in (20, 21, 33, 50):
+        p, _ = make("recovery_nuclei", tmp_path, tmax=repr(float(0.5 * (t[k - 1] + t[k]))))
+        ref = oracle.run(p, d)
+        assert len(ref["trace"]) == k + 1
+        for lim in ({"host_polls": 1}, {"host_polls": 1, "slots": 500}, {}):
+            tr, labels, counts, _ = run(p, d, **lim)
+            assert_same(tr, labels, *counts, ref)
