@@ -697,6 +697,9 @@ constexpr uint64_t kFuseBlockSlots = 200ull << 10;
 // 42 us a step with 2, 23 with 4), but half the tiles to spread over the blocks.
 constexpr uint64_t kFuseWide = 4096;
 
+// A launch's turn, after which its groups leave so that other work of the device gets its own.
+constexpr int64_t kFuseTurnUs = 2000;
+
 // The limits of an engine's fused steps.  Results do not depend on them: tests lower them, so that small domains take
 // every path (score_internal_step_limits), never raise them.
 struct StepLimits {
@@ -1935,6 +1938,9 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
     launches += 1;
     for (FuseServe& f : sv) f.c->fuse_replay = 0;
     std::atomic<bool> stop{false};
+    // the launch's turn starts with its first step: one that has waited in the queue for other work has not used any
+    std::atomic<int64_t> turn{0};
+    auto now_us = [&] { return std::chrono::duration_cast<std::chrono::microseconds>(std::chrono::steady_clock::now() - t0).count() + 1; };
     const double bpu = fp32 ? 21.0 : 25.0;
     const uint64_t sample0 = run_steps;
     auto timed_step = [&](const FuseServe& f) {
@@ -1989,6 +1995,10 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
             return true;
         }
         c->fuse_seq = fuse_next(seq);
+        if (turn.load(std::memory_order_relaxed) == 0) {
+            int64_t none = 0;
+            turn.compare_exchange_strong(none, now_us());
+        }
         const DevState& hs = c->h_box->snap;
         if (hs.err || hs.nmiss > kBoxMiss || hs.ndepleted > kBoxDep) {
             f.deferred = true;
@@ -2038,8 +2048,10 @@ int Engine::fused_session(double x_target, uint32_t max_steps, bool one, std::ve
             }
             if (!open) return;
             if (any) idle = 0;
-            if ((any || (++idle & 0xFFFu) == 0) && std::chrono::steady_clock::now() - t_pre > std::chrono::milliseconds(2))
-                stop.store(true, std::memory_order_relaxed);
+            if (any || (++idle & 0xFFFu) == 0) {
+                const int64_t since = turn.load(std::memory_order_relaxed);
+                if (since != 0 && now_us() - since > kFuseTurnUs) stop.store(true, std::memory_order_relaxed);
+            }
             if (any || (idle & 0xFFFFu) != 0) continue;
             // long silence: has the launch ended (an error, or a wait on the device that gave up)?
             const cudaError_t q = cudaStreamQuery(stream);
