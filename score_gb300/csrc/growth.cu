@@ -2537,7 +2537,9 @@ int score_load_domain(score_ctx* c, const uint32_t* grid, const double* defg_qua
         if (e == cudaSuccess) e = dalloc(&a.rxg_cnt, nrxg);
         if (e == cudaSuccess) e = dalloc(&a.depleted, ndefg);
         if (e == cudaSuccess) e = dalloc(&a.miss, a.misscap);
-        a.touchcap = std::min<uint32_t>(a.misscap, 1u << 22);
+        // a restart clears the listed entries up to 1/64 of the table, else all of it: no more than that is listed, and no more
+        // than 8 MB (a 512^3 run lists 0.3 M entries)
+        a.touchcap = (uint32_t)std::min<uint64_t>({a.misscap, ptab_words / 64 + 1, 1ull << 20});
         if (e == cudaSuccess) e = dalloc(&a.touched, a.touchcap);
         if (e == cudaSuccess) e = dalloc((float4**)&a.rxq, nrxg);
         if (e == cudaSuccess) e = dalloc((float4**)&a.dfq, ndefg);
