@@ -908,8 +908,9 @@ double weight_of(score_ctx* c, uint32_t r, uint32_t g) {
     return mobility_weight(c->prm, &c->rxg_q[4 * (size_t)r], &c->defg_q[4 * (size_t)g]);
 }
 
-// thresholds of the FP32 classification (weight_class)
-WeightClass make_weight_class(const score_params& p) {
+// thresholds of the FP32 classification (weight_class), for the weight as the host computes it or as the table does, which
+// takes the second disorientation at any angle
+WeightClass make_weight_class(const score_params& p, bool table = false) {
     double fac = 0, lagb = 0, maxdev = 0, m40[4], sat = 0;
     weight_constants(p, &fac, &lagb, &maxdev, m40, &sat);
     WeightClass w{};
@@ -920,6 +921,7 @@ WeightClass make_weight_class(const score_params& p) {
     w.cos_hi = (float)std::cos(0.5 * (deg40 + maxdev));
     w.cos_dev = (float)std::cos(0.5 * maxdev);
     w.cos_sat = sat < kPi ? (float)std::cos(0.5 * sat) : -2.0f;
+    w.far_norm = table ? kWeightUnit : 1.0f;
     for (int i = 0; i < 4; ++i) w.m40[i] = (float)m40[i];
     return w;
 }
@@ -3212,7 +3214,7 @@ extern "C" int score_mobility_table_noalloc(const score_params* p, const double*
     t.rh_cut = p->RH_cut;
     t.rh_trans = p->RH_trans;
     t.rh_expo = p->RH_exponent;
-    t.cls = make_weight_class(*p);
+    t.cls = make_weight_class(*p, true);
     cudaStream_t st = (cudaStream_t)stream;
     // the completion counter starts at 0 whatever an earlier launch left behind
     if (cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), st) != cudaSuccess) return SCORE_ERR_CUDA;

@@ -91,6 +91,7 @@ struct WeightClass {            // what the classification needs of the paramete
     float cos_lo, cos_hi;       // cos of half of 30 and 50 deg: |angle - 40 deg| beyond 10 deg needs no axis
     float cos_dev;              // cos(5 deg)
     float cos_sat;              // cos of half the angle from which the sigmoid is exactly 1
+    float far_norm;             // |n|^2 - 1 up to which the angle alone says "far from 40 deg <111>"
     float m40[4];               // 40 deg <111>
 };
 
@@ -1574,7 +1575,11 @@ __device__ __forceinline__ double d_disori(const DomainArgs& A, const double p[4
 // factors rounded to 24 bits and 3 sums, below 7e-7; a candidate sums 2 (times sqrt(1/2)) or 4 (times 1/2)
 // of them, below 1.5e-6; the second product has factors off by that much, its candidates below 1.3e-5.
 // The margins are five times that.
-constexpr float kWeightEps = 8e-6f, kWeightEps2 = 7e-5f;
+// That a pair more than 10 deg from 40 deg is as far from 40 deg <111> holds for unit quaternions.  Of length 1 + d the angle
+// beside the threshold moves by 2 d / tan 15 deg, and the second disorientation with it: the weight is 0 with both
+// as long as d < .2548 (margin - 1.5e-6), 4.7e-6 with kWeightEpsFar; the squared length is within 3.1e-6, so pairs up
+// to kWeightUnit take the short way (d < 3.6e-6).  The host's weight takes it whatever the length.
+constexpr float kWeightEps = 8e-6f, kWeightEps2 = 7e-5f, kWeightEpsFar = 2e-5f, kWeightUnit = 4e-6f;
 constexpr int kWeightUnknown = 2;
 
 // the largest component of each of the six symmetry families of (a, b, c, d), as d_grimmer orders them
@@ -1615,7 +1620,7 @@ __device__ __noinline__ int weight_class(const WeightClass& w, float4 rx, float4
     if (om > w.cos_lagb + kWeightEps) return -1;
     if (!(om < w.cos_lagb - kWeightEps)) return kWeightUnknown;
     // the deviation from 40 deg <111> is at least the difference of the angles
-    if (om > w.cos_lo + kWeightEps || om < w.cos_hi - kWeightEps) return 0;
+    if ((om > w.cos_lo + kWeightEpsFar || om < w.cos_hi - kWeightEpsFar) && fabsf(n2 - 1.0f) <= w.far_norm) return 0;
     if (!(om - om2 > 2.0f * kWeightEps)) return kWeightUnknown;  // the best candidate could be another one
     float s[4];
     if (mi == 5) {
