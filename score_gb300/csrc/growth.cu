@@ -524,14 +524,7 @@ struct score_ctx {
         err = std::string(what) + ": " + cudaGetErrorString(e);
         return SCORE_ERR_CUDA;
     }
-    bool stage(size_t bytes) {
-        if (bytes <= stage_cap) return true;
-        if (d_stage) cudaFree(d_stage);
-        d_stage = nullptr; stage_cap = 0;
-        if (cudaMalloc(&d_stage, bytes) != cudaSuccess) return false;
-        stage_cap = bytes;
-        return true;
-    }
+    bool stage(size_t bytes);
 };
 
 void score_ctx::release_domain() {
@@ -700,14 +693,15 @@ constexpr uint64_t kFuseWide = 4096;
 // A launch's turn, after which its groups leave so that other work of the device gets its own.
 constexpr int64_t kFuseTurnUs = 2000;
 
-// The limits of an engine's fused steps.  Results do not depend on them: tests lower them, so that small domains take
-// every path (score_internal_step_limits), never raise them.
+// The limits of an engine's fused steps and staging.  Results do not depend on them: tests lower them, so that small domains
+// take every path (score_internal_step_limits), never raise them.
 struct StepLimits {
     uint32_t host_polls = kFuseHostSpin, group_polls = kFuseSpin;
     uint32_t wide = (uint32_t)kFuseWide, block_slots = (uint32_t)kFuseBlockSlots;
     uint64_t slots = kFuseSlots;
     uint32_t number = 0;               // of the next command (1 to kCmdSeqMask; 0: as it is)
     uint32_t refuse_after = ~0u;       // cooperative launches until one is answered as refused (~0: never)
+    uint64_t stage = ~0ull;            // bytes beyond which a staging buffer is refused
 };
 
 struct Engine {
@@ -829,6 +823,20 @@ void for_grains(score_ctx* c, Body body) {
     E.pool->run(kChunks, [&](int k) { body(n * (size_t)k / kChunks, n * (size_t)(k + 1) / kChunks); });
 }
 }  // namespace
+
+bool score_ctx::stage(size_t bytes) {
+    if (bytes <= stage_cap) return true;
+    if (bytes > eng->lim.stage) return false;
+    if (d_stage) cudaFree(d_stage);
+    d_stage = nullptr; stage_cap = 0;
+    if (cudaMalloc(&d_stage, bytes) != cudaSuccess) {
+        cudaGetLastError();  // the caller may go on without
+        d_stage = nullptr;
+        return false;
+    }
+    stage_cap = bytes;
+    return true;
+}
 
 // (after Engine is complete: deleting it runs its destructor, which returns its
 // argument slots, stream, events and pinned buffers)
@@ -1167,10 +1175,8 @@ int reset_state(score_ctx* c) {
                 c->launches++;
                 e = cudaGetLastError();
             }
-        }
-        if (e == cudaSuccess && nt && !(c->ptab_dirty_all || nt + c->ntouch > total / 64)) {
-            e = cudaMemcpyAsync(c->d_stage, c->ptab_touched.data(), nt * 8, cudaMemcpyHostToDevice, st);
-            if (e == cudaSuccess) {
+            if (e == cudaSuccess && nt) e = cudaMemcpyAsync(c->d_stage, c->ptab_touched.data(), nt * 8, cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess && nt) {
                 k_clear_ptab<<<blocks_for(nt, c->sms), kBlock, 0, st>>>(a.ptab, (const unsigned long long*)c->d_stage, (uint32_t)nt);
                 c->launches++;
                 e = cudaGetLastError();
@@ -3005,6 +3011,7 @@ StepLimits lowered(const StepLimits* l) {
     r.block_slots = std::min(l->block_slots, d.block_slots);
     r.slots = std::min(l->slots, d.slots);
     r.refuse_after = l->refuse_after;
+    r.stage = l->stage;
     return r;
 }
 }  // namespace
