@@ -525,6 +525,10 @@ struct score_ctx {
         return SCORE_ERR_CUDA;
     }
     bool stage(size_t bytes);
+    void unstage() {
+        if (d_stage) cudaFree(d_stage);
+        d_stage = nullptr; stage_cap = 0;
+    }
 };
 
 void score_ctx::release_domain() {
@@ -827,8 +831,7 @@ void for_grains(score_ctx* c, Body body) {
 bool score_ctx::stage(size_t bytes) {
     if (bytes <= stage_cap) return true;
     if (bytes > eng->lim.stage) return false;
-    if (d_stage) cudaFree(d_stage);
-    d_stage = nullptr; stage_cap = 0;
+    unstage();
     if (cudaMalloc(&d_stage, bytes) != cudaSuccess) {
         cudaGetLastError();  // the caller may go on without
         d_stage = nullptr;
@@ -2306,6 +2309,10 @@ int grainevo_get(score_ctx* c, uint32_t i, score_grainevo_info* info, uint32_t* 
     return SCORE_OK;
 }
 
+// Rows of k_rediscr_rows held at a time: the domains go in groups of up to kRowBytes (one at least), and a staging buffer larger
+// than kRowKeep goes back after the call.
+constexpr size_t kRowBytes = 256u << 20, kRowKeep = 64u << 20;
+
 // Ensemble post-processing of the domains' grain-evolution logs on the device: kinetics (cls null)
 // or macrotexture by orientation class.  Writes the time slots and [slot] or [slot][class] sums.
 int rediscr(const std::vector<score_ctx*>& doms, uint32_t nslots, const uint32_t* cls, uint32_t nclass, double* t_out,
@@ -2336,12 +2343,18 @@ int rediscr(const std::vector<score_ctx*>& doms, uint32_t nslots, const uint32_t
     const uint32_t ndom = (uint32_t)doms.size(), m = cls ? nslots * nclass : nslots, nc = cls ? nclass : 1u;
     // one block of the first domain's staging buffer: what the host sends (descriptors, snapshot times, slot times,
     // grains by class), then rows and sums
-    size_t nrows = 0, maxgr = 0;
-    for (score_ctx* c : doms) {
-        const size_t ngr = cls ? (size_t)c->ndefg + c->nrxg : c->ndefg;
-        nrows += (c->log_info.size() + 2) * ngr;
-        maxgr = std::max(maxgr, ngr);
+    auto ngr_of = [&](const score_ctx* c) { return cls ? (size_t)c->ndefg + c->nrxg : (size_t)c->ndefg; };
+    auto rows_of = [&](const score_ctx* c) { return (c->log_info.size() + 2) * ngr_of(c); };
+    std::vector<uint32_t> group(1, 0);  // first domain of each group, and the end
+    size_t nrows = 0, in_group = 0, maxgr = 0;
+    for (uint32_t d = 0; d < ndom; ++d) {
+        const size_t r = rows_of(doms[d]);
+        if (d > group.back() && (in_group + r) * 16 > kRowBytes) { group.push_back(d); in_group = 0; }
+        in_group += r;
+        nrows = std::max(nrows, in_group);
+        maxgr = std::max(maxgr, ngr_of(doms[d]));
     }
+    group.push_back(ndom);
     const size_t b_evo = ndom * sizeof(EvoDev), b_t = ntimes * 8, b_w = (size_t)nslots * 8, b_o = cls ? ncls * 4 : 0, b_f = cls ? (size_t)ndom * (nc + 1) * 4 : 0;
     const size_t b_pd = (size_t)ndom * m * 8, b_out = (size_t)m * 8;
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -2365,7 +2378,7 @@ int rediscr(const std::vector<score_ctx*>& doms, uint32_t nslots, const uint32_t
         v.fin_defg = c->a.defg_cnt;
         v.fin_rxg = c->a.rxg_cnt;
         v.ndefg = c->ndefg; v.nrxg = c->nrxg; v.nsnap = (uint32_t)c->log_info.size();
-        v.ngr = cls ? G : c->ndefg;
+        v.ngr = (uint32_t)ngr_of(c);
         v.tsimend = c->ph.t; v.nboxvol = (double)c->N;
         if (cls) {  // grains by class, in grain order within a class
             v.order = (const uint32_t*)(blk + o_o) + coff;
@@ -2378,26 +2391,34 @@ int rediscr(const std::vector<score_ctx*>& doms, uint32_t nslots, const uint32_t
             for (uint32_t k = 0; k < nc; ++k) at[k] = f[k];
             for (uint32_t g = 0; g < G; ++g) order[coff + at[cls[coff + g]]++] = g;
         }
+        if (std::find(group.begin(), group.end(), d) != group.end()) roff = 0;
         v.rows = (double2*)(blk + sent) + roff;
         for (const auto& info : c->log_info) times[toff++] = info.t;
         coff += G;
-        roff += ((size_t)v.nsnap + 2) * v.ngr;
+        roff += rows_of(c);
         evo[d] = v;
     }
     cudaStream_t st = doms[0]->stream;
     cudaError_t e = cudaMemcpyAsync(blk, host.data(), sent, cudaMemcpyHostToDevice, st);
     double* const d_pd = (double*)(blk + o_pd);
     double* const d_out = (double*)(blk + o_out);
+    for (size_t k = 0; k + 1 < group.size() && e == cudaSuccess; ++k) {
+        const uint32_t d0 = group[k], nd = group[k + 1] - d0;
+        const EvoDev* d_evo = (const EvoDev*)blk + d0;
+        k_rediscr_rows<<<dim3((unsigned)((maxgr + 255) / 256), nd), 256, 0, st>>>(d_evo);
+        k_rediscr_sum<<<dim3((nslots + 31) / 32, nc, nd), 32, 0, st>>>(d_evo, (const double*)(blk + o_w), nslots, nc, cls ? 0 : 1,
+                                                                       d_pd + (size_t)d0 * m);
+        doms[0]->launches += 2;
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess) {
-        const EvoDev* d_evo = (const EvoDev*)blk;
-        k_rediscr_rows<<<dim3((unsigned)((maxgr + 255) / 256), ndom), 256, 0, st>>>(d_evo);
-        k_rediscr_sum<<<dim3((nslots + 31) / 32, nc, ndom), 32, 0, st>>>(d_evo, (const double*)(blk + o_w), nslots, nc, cls ? 0 : 1, d_pd);
         k_rediscr_ensemble<<<(m + 127) / 128, 128, 0, st>>>(d_pd, ndom, m, d_out);
-        doms[0]->launches += 3;
+        doms[0]->launches++;
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, b_out, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (doms[0]->stage_cap > kRowKeep) doms[0]->unstage();
     if (e != cudaSuccess) { err = std::string("post-processing: ") + cudaGetErrorString(e); return SCORE_ERR_CUDA; }
     return SCORE_OK;
 }

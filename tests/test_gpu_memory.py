@@ -1,4 +1,5 @@
 """Device memory of a loaded domain and of post-processing: no list or workspace beyond what the domain's arrays take."""
+import numpy as np
 import pytest
 
 import oracle
@@ -56,3 +57,34 @@ def test_restart_without_a_staging_buffer(gpu, tmp_path):
         set_limits(gm)
         gm.place_nuclei()
         assert_same(gm.run_until(), gm.labels(), *gm.grain_counts(), ref)
+
+
+def test_postprocessing_rows(gpu, tmp_path):
+    """Six domains of 20,000 grains and up to 256 snapshots, some 400 MB of slopes: in groups, the sums the oracle's, and no
+    large buffer kept after the call."""
+    n = 48
+    logs = [repr(round(0.0037 * k, 6)) for k in range(1, 257)]
+    p = sg.read_uds(sg.UdsSpec(nx=n, ny=n, nz=n, logpoints=logs, border_policy=1).write(tmp_path / "p.uds"))
+    doms = [sg.generate_domain(n, n, n, 20000, 24, seed=40 + k, device=0) for k in range(6)]
+    with sg.Batch([p] * len(doms)) as b:
+        for k, d in enumerate(doms):
+            b.load_domain(k, d)
+        b.place_nuclei()
+        b.run_until()
+        evo = []
+        for k, d in enumerate(doms):
+            log = b.grainevo(k)
+            rx, deformed = b.grain_counts(k)
+            evo.append({"ndefg": d.ndefg, "nrxg": d.nrxg, "t": np.array([x[0].t for x in log]), "counts": np.array([x[1] for x in log]),
+                        "final": np.concatenate([deformed, rx]), "tsimend": b.stats(k).t, "cells": d.ncells,
+                        "cls": (np.arange(d.ndefg + d.nrxg) % 3).astype(np.uint32)})
+        assert sum((len(e["t"]) + 2) * e["ndefg"] * 16 for e in evo) > 300 * 2**20
+        before = used()
+        t, v, box = b.rediscr_kinetics(40)
+        t2, v2 = b.rediscr_texture(40, np.concatenate([e["cls"] for e in evo]), 3)
+        after = used()
+        t0, v0, box0 = oracle.rediscr_kinetics(evo, 40)
+        assert np.array_equal(t, t0) and np.array_equal(v, v0) and box == box0
+        t0, v0 = oracle.rediscr_texture(evo, 40, 3)
+        assert np.array_equal(t2, t0) and np.array_equal(v2, v0)
+        assert after - before <= 72 * 2**20, "a large buffer was kept"
