@@ -774,7 +774,7 @@ def main():
                     "phase_sampling": f"device phases (grow, fill, claim, commit) timed with CUDA events on {timed_steps} "
                                       f"of {grow_launches} steps (every {every}th) and scaled to the runs; "
                                       f"roofline over the timed fill launches; host phases every step",
-                    "host_weight_misses_per_run": wl.misses})
+                    "weight_pairs_met_per_run": wl.misses})
         if wl.tuned is not None:
             t = wl.tuned
             cfg["autotuned"] = {"items": t.items, "fill_blocks_per_sm": t.fill_blocks_per_sm,

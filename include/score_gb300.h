@@ -131,7 +131,8 @@ typedef struct score_step_stats {
     double dXstep;        /* sum of fill increments (observation; order differs from the reference) */
     uint32_t next_never[2];  /* Inside, Border: slots ever used */
     uint32_t n_recycled[2];  /* Inside, Border: recycle-list lengths this step */
-    uint32_t p_misses;       /* mobility weights computed on the host this step */
+    uint32_t p_misses;       /* (rx grain, deformed grain) pairs first met this step, their weight from the host or,
+                                where it is a constant, settled on the device */
     uint32_t reserved;
 } score_step_stats;
 
