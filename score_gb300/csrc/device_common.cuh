@@ -67,8 +67,8 @@ constexpr int8_t kStencilDy[26] = SCORE_STENCIL_DY;
 constexpr int8_t kStencilDz[26] = SCORE_STENCIL_DZ;
 // A direction in one word: dx + 1 | (dy + 1) << 2 | (dz + 1) << 4 | overshoot class << 6 | infector code << 8.  Kernels keep
 // the 26 words in shared memory: lanes of a warp that look at different directions make a constant load
-// one pass a direction (with seven such loads a new cell a recovering 384^3 front took 131.5 ms, without 129.0; a
-// 16-domain batch 59.3 and 58.4).
+// one pass a direction (with seven such loads a new cell a run of a recovering 384^3 domain took 132.6 ms, without 130.1;
+// sheets 168.5 and 166.4, a 16-domain batch 59.2 and 58.6).
 constexpr uint8_t kCode[26] = {16, 15, 14, 13, 12, 11, 10, 9, 19, 18, 17, 25, 24, 23, 22, 21, 20, 8, 7, 6, 5, 4, 3, 2, 1, 0};
 constexpr uint32_t dir_word(int d) {
     const int dx = kStencilDx[d], dy = kStencilDy[d], dz = kStencilDz[d];

@@ -738,8 +738,8 @@ __global__ void __launch_bounds__(kFuse, 1) k_steps_fused(const __grid_constant_
             }
         }
         // a thread takes one full cell a chunk: its grains and overshoot, and what needs no rank, the first chunk's before
-        // the barrier, whose wait hides the loads and the atomics' answers (after it: 4.7 us a step of the
-        // commit on the 64^3 domain, now 4.0; a 384^3 front of sheets 95.8 us a step, now 93.2)
+        // the barrier, whose wait hides the loads and the atomics' answers (a run of a recovering 384^3 domain 135.3 ms with
+        // them after it, 132.4 before; sheets 170.7 and 168.4; 64^3 10.2 and 10.3)
         FullCell fc;
         take_full<FP32>(cst, a, rec, threadIdx.x, F, fc);
         __syncthreads();

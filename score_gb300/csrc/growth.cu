@@ -139,7 +139,7 @@ __global__ void k_fill_ptab(unsigned long long* ptab, const unsigned long long* 
         ptab[idx[i]] = (unsigned long long)__double_as_longlong(val[i]);
 }
 
-// new cells whose P arrived from the host: their velocity factor
+// labels of the front's cells by the clarify rule (half filled: the rx grain) into the linear map
 template <bool FP32>
 __global__ void k_labels_front(DomainArgs a, int L, uint32_t n, uint32_t* lab) {
     const DFront& f = a.f[L];
@@ -565,7 +565,7 @@ struct TuneCfg {
     int items = 8;          // grow tile = kBlock * items slots
     int fill_bpsm = 16;     // k_grow_fill blocks per SM
     int claim_bpsm = 4;     // k_claim blocks per SM: what fits at 64 registers
-    int commit_bpsm = 8;    // k_resolve / k_commit blocks per SM (same)
+    int commit_bpsm = 8;    // k_resolve / k_commit blocks per SM (autotuner's choice on the 512^3 workload)
     int spec_pct = 30;      // every slot's data loaded with its infector byte up to this INACTIVE share [%]
     int timing_every = 8;   // phase events on every k-th step of a run (0 never): each event costs
                             // microseconds of device time, so the steps in between run without
@@ -1464,7 +1464,7 @@ int post_step(score_ctx* c, uint32_t newnuc, score_step_stats* out) {
     o.Pmax = ph.Pmax; o.rhomax = rhomax_step; o.dXstep = 0.0;
     o.next_never[0] = c->next_never[0]; o.next_never[1] = c->next_never[1];
     o.n_recycled[0] = hs.nrec[0]; o.n_recycled[1] = hs.nrec[1];
-    o.p_misses = nreq + hs.nknown;  // pairs met first in this step
+    o.p_misses = nreq + hs.nknown;
     if (out) *out = o;
     return SCORE_OK;
 }
@@ -2782,7 +2782,8 @@ int score_autotune(score_ctx* c, double x_target, uint32_t max_steps, score_tune
 // A batch splits its domains into groups of about equal cell count, each stepped by its own
 // engine (stream, argument slots, graphs, workers) from its own host thread: the groups'
 // latency-bound kernels overlap on the GPU and their host work overlaps on the CPU.  Within a
-// group the domains step in lock-step, one sequence of launches per step.
+// group small fronts step inside one launch, each domain at its own pace (k_steps_fused); larger ones step
+// together, one sequence of launches per step.
 struct score_batch {
     std::vector<std::unique_ptr<Engine>> engs;
     std::vector<score_ctx*> dom;

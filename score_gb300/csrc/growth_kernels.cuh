@@ -195,8 +195,8 @@ __device__ __forceinline__ bool target_of(const DomainArgs& a, int L, int x, int
 // mobility m(P) of the reference (get_currentintrinsicmobility, SCORE_Kernel.cpp:5459-5470)
 __device__ __forceinline__ double mobility(const DomainArgs& a, double P) {
     // the constants by integers (FP64, compares included, runs at 1/64 rate): 94 % of the pairs.  0 mGS + 1 mHAGB is
-    // mHAGB and 1 mGS + 0 mHAGB is mGS where both are finite and not negative (384^3 sheets 61.4 ms, now 60.6; 64^3
-    // 13.2, now 13.1)
+    // mHAGB and 1 mGS + 0 mHAGB is mGS where both are finite and not negative.  Runs alone, whose medians repeat within 0.3 %:
+    // 384^3 sheets 166.6 ms without, 165.4 with; 512^3 103.1 and 102.7; others the same
     const unsigned long long b = (unsigned long long)__double_as_longlong(P);
     if (a.mobility_model == 2) return b == 0x3FF0000000000000ull ? a.mRH : __dmul_rn(P, a.mRH);
     if (b > 0x8000000000000000ull && b <= 0xFFF0000000000000ull) return a.mLAGB;  // P < 0
