@@ -919,9 +919,8 @@ double weight_of(score_ctx* c, uint32_t r, uint32_t g) {
     return mobility_weight(c->prm, &c->rxg_q[4 * (size_t)r], &c->defg_q[4 * (size_t)g]);
 }
 
-// thresholds of the FP32 classification (weight_class), for the weight as the host computes it or as the table does, which
-// takes the second disorientation at any angle
-WeightClass make_weight_class(const score_params& p, bool table = false) {
+// thresholds of the FP32 classification (weight_class)
+WeightClass make_weight_class(const score_params& p) {
     double fac = 0, lagb = 0, maxdev = 0, m40[4], sat = 0;
     weight_constants(p, &fac, &lagb, &maxdev, m40, &sat);
     WeightClass w{};
@@ -932,7 +931,6 @@ WeightClass make_weight_class(const score_params& p, bool table = false) {
     w.cos_hi = (float)std::cos(0.5 * (deg40 + maxdev));
     w.cos_dev = (float)std::cos(0.5 * maxdev);
     w.cos_sat = sat < kPi ? (float)std::cos(0.5 * sat) : -2.0f;
-    w.far_norm = table ? kWeightUnit : 1.0f;
     for (int i = 0; i < 4; ++i) w.m40[i] = (float)m40[i];
     return w;
 }
@@ -3146,7 +3144,7 @@ __global__ void __launch_bounds__(kTableCols) k_mobility_table(TableArgs t, cons
             const double* q = dfq + 4 * (size_t)j;
             const float4 df = make_float4((float)q[0], (float)q[1], (float)q[2], (float)q[3]);
             for (uint32_t r = 0; r < rows; ++r) {
-                const int c = weight_class(t.cls, s_rx[r], df);
+                const int c = weight_class<true>(t.cls, s_rx[r], df);
                 if (c == kWeightUnknown) {
                     s_q[atomicAdd(&s_n, 1u)] = (uint16_t)((r << 8) | threadIdx.x);
                 } else {
@@ -3243,7 +3241,7 @@ extern "C" int score_mobility_table_noalloc(const score_params* p, const double*
     t.rh_cut = p->RH_cut;
     t.rh_trans = p->RH_trans;
     t.rh_expo = p->RH_exponent;
-    t.cls = make_weight_class(*p, true);
+    t.cls = make_weight_class(*p);
     cudaStream_t st = (cudaStream_t)stream;
     // the completion counter starts at 0 whatever an earlier launch left behind
     if (cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), st) != cudaSuccess) return SCORE_ERR_CUDA;

@@ -91,7 +91,6 @@ struct WeightClass {            // what the classification needs of the paramete
     float cos_lo, cos_hi;       // cos of half of 30 and 50 deg: |angle - 40 deg| beyond 10 deg needs no axis
     float cos_dev;              // cos(5 deg)
     float cos_sat;              // cos of half the angle from which the sigmoid is exactly 1
-    float far_norm;             // |n|^2 - 1 up to which the angle alone says "far from 40 deg <111>"
     float m40[4];               // 40 deg <111>
 };
 
@@ -1600,7 +1599,9 @@ __device__ __forceinline__ void misorientation(const float p[4], const float q[4
     r[2] = p[2] * q[0] - p[0] * q[2] + q[1] * p[3] - q[3] * p[1];
     r[3] = p[3] * q[0] - p[0] * q[3] - q[1] * p[2] + q[2] * p[1];
 }
-// -1, 0 or 1: the weight is that constant; kWeightUnknown: too close to a threshold, or not a constant
+// -1, 0 or 1: the weight is that constant; kWeightUnknown: too close to a threshold, or not a constant.  TABLE: of the weight as
+// the table computes it, else as the host does
+template <bool TABLE>
 __device__ __noinline__ int weight_class(const WeightClass& w, float4 rx, float4 df) {
     const float p[4] = {rx.x, rx.y, rx.z, rx.w}, q[4] = {df.x, df.y, df.z, df.w};
     float r[4], f[6];
@@ -1620,7 +1621,7 @@ __device__ __noinline__ int weight_class(const WeightClass& w, float4 rx, float4
     if (om > w.cos_lagb + kWeightEps) return -1;
     if (!(om < w.cos_lagb - kWeightEps)) return kWeightUnknown;
     // the deviation from 40 deg <111> is at least the difference of the angles
-    if ((om > w.cos_lo + kWeightEpsFar || om < w.cos_hi - kWeightEpsFar) && fabsf(n2 - 1.0f) <= w.far_norm) return 0;
+    if ((om > w.cos_lo + kWeightEpsFar || om < w.cos_hi - kWeightEpsFar) && (!TABLE || fabsf(n2 - 1.0f) <= kWeightUnit)) return 0;
     if (!(om - om2 > 2.0f * kWeightEps)) return kWeightUnknown;  // the best candidate could be another one
     float s[4];
     if (mi == 5) {
@@ -1664,7 +1665,7 @@ __device__ __forceinline__ bool lookup_p(const DomainArgs& a, uint32_t rxg, uint
     // a stale EMPTY is settled by the compare-and-swap below
     unsigned long long bits = *e;
     if (bits == kPtabEmpty) {
-        const int c = weight_class(a.cls, a.rxq[rxg], a.dfq[defg]);
+        const int c = weight_class<false>(a.cls, a.rxq[rxg], a.dfq[defg]);
         if (c != kWeightUnknown) {
             P = __hiloint2double(c == 0 ? 0 : c < 0 ? (int)0xBFF00000u : 0x3FF00000, 0);
             if (atomicCAS(e, kPtabEmpty, (unsigned long long)__double_as_longlong(P)) == kPtabEmpty) {
