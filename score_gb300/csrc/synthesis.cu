@@ -91,10 +91,11 @@ __device__ __forceinline__ uint32_t bucket_cell(uint32_t b, uint32_t nb, uint32_
     return c <= 0.0 ? 0u : min(n, (uint32_t)c);
 }
 
-// Block (bucket, part): the part's share of the bucket's cells, 256 at a time.  FP32 error of a squared distance
-// D^2 (scaled): a seed's position relative to the bucket is rounded once (2^-24 of its size, at most the
-// domain's largest edge) and the difference once, so a component is off by at most 2 u, u = 2^-24 edge, in
-// units of its scale, D^2 by 2 D sqrt(3) 2 u / scale + 6e-7 D^2; `tol` takes twice that.
+// Block (bucket, part): the part's share of the bucket's cells, 256 at a time.  Distances in FP32 are in units of the finest
+// axis' scale, so that their squares stay in range whatever the scales.  Error of a squared distance D^2: a
+// seed's position relative to the bucket is rounded once (2^-24 of its size, at most the domain's largest
+// edge), the cell's twice and the difference once, so a component is off by at most e = 4 u, u = 2^-24 edge, D^2 by
+// 2 sqrt(3) e D + 3 e^2 + 6e-7 D^2; `tol` is above that.
 __global__ void __launch_bounds__(256) k_voronoi_fill(VoronoiDev v, uint32_t parts, uint32_t* grid) {
     __shared__ float4 s_seed[kSeedCap];  // position relative to the bucket's first cell, id
     __shared__ uint32_t s_n;
@@ -110,9 +111,10 @@ __global__ void __launch_bounds__(256) k_voronoi_fill(VoronoiDev v, uint32_t par
     }
     const uint64_t M = (uint64_t)w[0] * w[1] * w[2];
     const uint64_t m_end = M * (blockIdx.y + 1) / parts;
-    const float inv[3] = {(float)(1.0 / v.scale[0]), (float)(1.0 / v.scale[1]), (float)(1.0 / v.scale[2])};
+    const double fine = fmin(v.scale[0], fmin(v.scale[1], v.scale[2]));
+    const float inv[3] = {(float)(fine / v.scale[0]), (float)(fine / v.scale[1]), (float)(fine / v.scale[2])};
     const float edge = (float)max(v.n[0], max(v.n[1], v.n[2]));
-    const float tol1 = 16.0f * 5.9604645e-8f * edge * fmaxf(inv[0], fmaxf(inv[1], inv[2])), tol2 = 1.5e-6f;
+    const float u = 5.9604645e-8f * edge, tol0 = 64.0f * u * u, tol1 = 16.0f * u, tol2 = 1.5e-6f;
     int have = 0;  // radius of the seeds in shared memory
     for (uint64_t m0 = M * blockIdx.y / parts; m0 < m_end; m0 += 256) {
         const uint64_t m = m0 + threadIdx.x;
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(256) k_voronoi_fill(VoronoiDev v, uint32_t par
                     if (d < best) { second = best; best = d; at = k; }
                     else second = fminf(second, d);
                 }
-                const float tol = tol1 * sqrtf(best) + tol2 * best;
+                const float tol = tol0 + tol1 * sqrtf(best) + tol2 * best;
                 // every seed not in the list lies beyond the slab of buckets along some axis
                 float lb = 3.0e38f;
 #pragma unroll
