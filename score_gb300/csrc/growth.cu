@@ -3246,7 +3246,7 @@ extern "C" int score_mobility_table_noalloc(const score_params* p, const double*
     // the completion counter starts at 0 whatever an earlier launch left behind
     if (cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), st) != cudaSuccess) return SCORE_ERR_CUDA;
     // rows a block: as many as leave the SMs two blocks each, so that a small table's chains run side by side
-    // (75 x 128 pairs: 22 us with one row a block, 28 with eight; 2000 x 1500: 174 us with eight)
+    // (75 x 128 pairs: 22 us with one row a block, 28 with eight; 2000 x 1500: 154 us with eight)
     const uint32_t gy = std::min((ndefg + kTableCols - 1) / kTableCols, kTableGridY);
     const uint32_t per = (uint32_t)std::min<uint64_t>(kTableRows, std::max<uint64_t>({1, (uint64_t)nrxg * gy / 304, (nrxg * gy + kTableMaxRows - 1) / kTableMaxRows}));
     // the launch's own status (not cudaGetLastError, which would also report, and clear,
