@@ -198,3 +198,46 @@ def test_stop_rules_wait_for_the_pending_step(gpu, tmp_path):
         for lim in ({"host_polls": 1}, {"host_polls": 1, "slots": 500}, {}):
             tr, labels, counts, _ = run(p, d, **lim)
             assert_same(tr, labels, *counts, ref)
+
+
+@pytest.mark.parametrize("kind", ["requests", "depleted"])
+def test_more_than_the_mailbox_holds(gpu, tmp_path, kind):
+    """A step that asks for more than 16,384 weights, or in which more deformed grains than that lose their last cell, is finished
+    after its launch."""
+    if kind == "requests":
+        n, par = 80, {"mobility_model": 2, "RH_exponent": "1.0"}
+        d = sg.generate_domain(n, n, n, 20000, 16000, seed=9, device=0)
+    else:
+        # cells of one front speed finish together, in grains of one or two cells
+        n, par = 64, {"mobility_model": 2}
+        d = sg.generate_domain(n, n, n, 250000, 6000, seed=9, device=0, rho_sigma=0.0)
+    p = sg.read_uds(sg.UdsSpec(nx=n, ny=n, nz=n, border_policy=1, **par).write(tmp_path / "p.uds"))
+    out = [run(p, d, use_graph=g) for g in (1, 0)]
+    tr = out[0][0]
+    assert out[0][3] < 5 * len(tr)
+    if kind == "requests":
+        assert max(s.p_misses for s in tr) > 16384
+        assert_same(*out[0][:2], *out[0][2], oracle.run(p, d))
+    else:
+        assert max(s.n_full for s in tr) > 40000
+    assert np.array_equal(as_array(tr), as_array(out[1][0])) and np.array_equal(out[0][1], out[1][1])
+    assert all(np.array_equal(a, b) for a, b in zip(out[0][2], out[1][2]))
+
+
+@pytest.mark.parametrize("polls", [1, 4096])
+def test_more_than_the_mailbox_holds_in_a_batch(gpu, tmp_path, polls):
+    """The others' pending answers move with those of the domain that overflows."""
+    n = 80
+    big = sg.read_uds(sg.UdsSpec(nx=n, ny=n, nz=n, border_policy=1, mobility_model=2, RH_exponent="1.0").write(tmp_path / "p.uds"))
+    cases = [(big, sg.generate_domain(n, n, n, 20000, 16000, seed=s, device=0)) for s in (9, 10)]
+    for name in ("odd_periodic", "heating_rh", "recovery_nuclei"):
+        cases.insert(1, make(name, tmp_path))
+    with sg.Batch([p for p, _ in cases]) as b:
+        set_limits(b, host_polls=polls)
+        for i, (_, d) in enumerate(cases):
+            b.load_domain(i, d)
+        b.place_nuclei()
+        b.run_until()
+        assert max(s.p_misses for s in b.trace(0)) > 16384
+        for i, (p, d) in enumerate(cases):
+            assert_same(b.trace(i), b.labels(i), *b.grain_counts(i), oracle.run(p, d))
