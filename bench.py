@@ -588,7 +588,7 @@ def measure_postprocessing(sg, local, doms, shapes, runs: int) -> dict:
                 "rediscr_kinetics_ms": 1e3 * kin, "rediscr_texture_ms": 1e3 * tex,
                 "interpolations_per_s_kinetics": 1000 * sum(d.ndefg for d in doms) / kin,
                 "interpolations_per_s_texture": 1000 * grains / tex,
-                "how": "host wall time of the public call (upload of the logs' times and classes, two kernels, download)"})
+                "how": "host wall time of the public call (upload of the logs' times and classes, three kernels, download)"})
     return out
 
 
